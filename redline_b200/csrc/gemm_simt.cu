@@ -3,74 +3,320 @@
 // This is the matrix product of the true 32-bit path (float operands, FFMA only,
 // no tensor-core or TF32 mode), and the fallback for any mix of float / bfloat16
 // operands (a weight stored in 32-bit next to bfloat16 activations, float logits
-// from bfloat16 operands at small sizes).  Any M, N, K.  The k loop runs in a
-// fixed order for every output element, so a row's result does not depend on how
-// many other rows are in the batch.
+// from bfloat16 operands at small sizes).  Any M, N, K.
+//
+// Every output is summed in one order, whichever kernel computes it and whatever else is in the batch: K is cut
+// into four quarters (of a multiple of four entries), a quarter's even and odd k run as two chains in ascending k
+// (the two halves of a packed fma.rn.f32x2, each rounded like a plain fma), even + odd is the quarter's sum, and the
+// quarters are added in order.  So a row's bits do not depend on how many other rows there are.  Places past the end
+// are zeros in both operands and leave a sum as it is.
+//
+// Two kernels.  Few rows are bound by the weights' way from DRAM, and want many thread blocks with deep copy
+// rings; many rows are bound by the FFMA pipe and want 8 x 8 outputs a thread, so that 16 shared-memory loads feed
+// 256 multiply-adds.
+// Measured on a B200 (float32; one launch over weights that are not in L2; in brackets the kernel of 64 x 64 tiles, 4 x 4
+// outputs a thread and one chain over all of K that stood here before):
+//   rows   N 3072 K 2048    N 2048 K 2048    N 16384 K 2048   N 2048 K 8192    N 128256 K 2048
+//      1    8.0 us (152)     6.7 us (151)     30 us (232)      22 us (602)      181 us (1181; 5.8 TB/s)
+//      4   12.2   (152)      8.1   (152)      38   (233)       30   (589)       221   (1191)
+//     16   22     (152)     21     (151)      66   (237)       77   (605)       437   (1226)
+//     64   50     (154)     33     (153)     149   (255)      127   (613)
+//    210  141     (303)     75     (210)     505   (690)      280   (626)
+//    512  219     (390)    147     (343)    1020  (1367)      557  (1214; 31 TFLOP/s)
+// Their error against float64 is a third of the one chain's (2.9e-7 against 8e-7 at K = 2048).
+#include <atomic>
+
 #include "common.cuh"
 
 namespace rl {
 
-constexpr int kTM = 64, kTN = 64, kTK = 16;
+constexpr int kQuarters = 4;
 
-template <typename TA, typename TW, typename TC>
-__global__ void __launch_bounds__(256)
-gemm_tn_simt_kernel(const TA* __restrict__ x, const TW* __restrict__ w, TC* __restrict__ y, int M,
-                    int N, int K, int ldx, int ldy) {
+__device__ __forceinline__ void fma2(unsigned long long& acc, unsigned long long a, unsigned long long b) {
+  asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc) : "l"(a), "l"(b));
+}
+__device__ __forceinline__ float even_plus_odd(unsigned long long acc) {
+  return __uint_as_float(static_cast<uint32_t>(acc)) + __uint_as_float(static_cast<uint32_t>(acc >> 32));
+}
+// 16 bytes to shared memory; zeros where `in` is false (src is then any valid address).
+__device__ __forceinline__ void copy16(void* dst, const void* src, bool in) {
+  const uint32_t d = static_cast<uint32_t>(__cvta_generic_to_shared(dst));
+  const int n = in ? 16 : 0;
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(src), "r"(n) : "memory");
+}
+__device__ __forceinline__ void commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void wait_group() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
+
+__host__ __device__ inline int quarter_len(int K) { return ((K + kQuarters - 1) / kQuarters + 3) & ~3; }
+
+// ---------------------------------------------------------------- few rows
+//
+// MG groups of 64 threads = 16 row groups x 4 quarters; a thread owns NPT weight rows of one quarter for MR rows of
+// x, every group other rows of x.  A stage brings 32 k of every quarter; segments are 36 floats apart, so that eight
+// neighbouring lanes' 16-byte reads fall into different banks.  N = 2048 gives 128 blocks (NPT = 1), which is what
+// fills the chip at the smallest products; the ring keeps about 50 KB on their way per SM.
+// Bound: the weights' bytes up to 2 rows; above, shared-memory reads (NPT + MR per NPT * MR * 4 multiply-adds), which
+// want more warps than two, hence the groups.
+constexpr int kSkK = 32, kSkPitch = kSkK + 4;
+
+template <int MR, int NPT, int MG, int STAGES>
+__global__ void __launch_bounds__(64 * MG)
+simt_few_kernel(const float* __restrict__ w, const float* x, float* y, int M, int N, int K, int ldx, int ldy) {
   pdl_launch();
-  pdl_wait();
-  __shared__ float xs[kTK][kTM + 4];
-  __shared__ float ws[kTK][kTN + 4];
-  const int m0 = blockIdx.y * kTM, n0 = blockIdx.x * kTN;
-  const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;  // 16 x 16 threads, 4 x 4 outputs each
-  const int lr = threadIdx.x >> 2, lk = (threadIdx.x & 3) * 4;  // loader: row 0..63, k offset 0,4,8,12
-  float acc[4][4];
-#pragma unroll
-  for (int i = 0; i < 4; ++i)
-#pragma unroll
-    for (int j = 0; j < 4; ++j) acc[i][j] = 0.f;
+  constexpr int kThreads = 64 * MG;
+  constexpr int NB = 16 * NPT;                     // weight rows of a block
+  constexpr int kWSegs = NB * kQuarters, kXSegs = MR * MG * kQuarters;
+  constexpr int kStageFloats = (kWSegs + kXSegs) * kSkPitch;
+  extern __shared__ __align__(16) float sm[];
+  const int t = threadIdx.x;
+  const int n0 = blockIdx.x * NB, m0 = blockIdx.y * (MR * MG);
+  const int ql = quarter_len(K);
+  const int steps = (ql + kSkK - 1) / kSkK;
 
-  for (int k0 = 0; k0 < K; k0 += kTK) {
+  auto ask_w = [&](int s) {
+    float* st = sm + (s % STAGES) * kStageFloats;
 #pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      const int k = k0 + lk + e;
-      const int m = m0 + lr, n = n0 + lr;
-      xs[lk + e][lr] = (m < M && k < K) ? to_float(x[static_cast<size_t>(m) * ldx + k]) : 0.f;
-      ws[lk + e][lr] = (n < N && k < K) ? to_float(w[static_cast<size_t>(n) * K + k]) : 0.f;
+    for (int j = 0; j < (kWSegs * 8 + kThreads - 1) / kThreads; ++j) {
+      const int c = j * kThreads + t, seg = c >> 3, piece = c & 7;
+      if (kWSegs * 8 % kThreads != 0 && seg >= kWSegs) break;
+      const int n = n0 + seg / kQuarters, q = seg % kQuarters;
+      const int off = s * kSkK + piece * 4, k = q * ql + off;
+      const bool in = n < N && off < ql && k < K;
+      copy16(st + seg * kSkPitch + piece * 4, in ? w + static_cast<size_t>(n) * K + k : w, in);
     }
-    __syncthreads();
-#pragma unroll
-    for (int k = 0; k < kTK; ++k) {
-      float a[4], b[4];
-#pragma unroll
-      for (int i = 0; i < 4; ++i) a[i] = xs[k][ty * 4 + i];
-#pragma unroll
-      for (int j = 0; j < 4; ++j) b[j] = ws[k][tx * 4 + j];
-#pragma unroll
-      for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(a[i], b[j], acc[i][j]);
+  };
+  auto ask_x = [&](int s) {
+    float* st = sm + (s % STAGES) * kStageFloats + kWSegs * kSkPitch;
+    for (int c = t; c < kXSegs * 8; c += kThreads) {
+      const int seg = c >> 3, piece = c & 7;
+      const int m = m0 + seg / kQuarters, q = seg % kQuarters;
+      const int off = s * kSkK + piece * 4, k = q * ql + off;
+      const bool in = m < M && off < ql && k < K;
+      copy16(st + seg * kSkPitch + piece * 4, in ? x + static_cast<size_t>(m) * ldx + k : x, in);
     }
-    __syncthreads();
+  };
+  // the weights are nobody's output: the ring is filled before the wait on the kernel before
+#pragma unroll
+  for (int s = 0; s < STAGES - 1; ++s)
+    if (s < steps) ask_w(s);
+  pdl_wait();
+#pragma unroll
+  for (int s = 0; s < STAGES - 1; ++s) {
+    if (s < steps) ask_x(s);
+    commit();                                      // (the weights asked for above belong to the first group)
   }
+  const int q = t % kQuarters, g = (t / kQuarters) % 16, mg = t / 64;  // lanes: four quarters of eight row groups
+  unsigned long long acc[NPT][MR];
 #pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const int m = m0 + ty * 4 + i;
-    if (m >= M) continue;
+  for (int i = 0; i < NPT; ++i)
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const int n = n0 + tx * 4 + j;
-      if (n < N) y[static_cast<size_t>(m) * ldy + n] = from_float<TC>(acc[i][j]);
+    for (int m = 0; m < MR; ++m) acc[i][m] = 0ull;
+
+  for (int s = 0; s < steps; ++s) {
+    wait_group<STAGES - 2>();
+    __syncthreads();
+    if (s + STAGES - 1 < steps) {
+      ask_w(s + STAGES - 1);
+      ask_x(s + STAGES - 1);
+    }
+    commit();
+    const float* st = sm + (s % STAGES) * kStageFloats;
+    const float* xs = st + (kWSegs + mg * MR * kQuarters + q) * kSkPitch;
+#pragma unroll
+    for (int p = 0; p < kSkK / 4; ++p) {
+      ulonglong2 a[NPT];
+#pragma unroll
+      for (int i = 0; i < NPT; ++i)
+        a[i] = *reinterpret_cast<const ulonglong2*>(st + ((i * 16 + g) * kQuarters + q) * kSkPitch + p * 4);
+#pragma unroll
+      for (int m = 0; m < MR; ++m) {
+        const ulonglong2 b = *reinterpret_cast<const ulonglong2*>(xs + m * kQuarters * kSkPitch + p * 4);
+#pragma unroll
+        for (int i = 0; i < NPT; ++i) {
+          fma2(acc[i][m], a[i].x, b.x);
+          fma2(acc[i][m], a[i].y, b.y);
+        }
+      }
+    }
+  }
+  // four neighbouring lanes hold an output's quarters
+#pragma unroll
+  for (int i = 0; i < NPT; ++i) {
+    const int n = n0 + i * 16 + g;
+#pragma unroll
+    for (int m = 0; m < MR; ++m) {
+      const int row = m0 + mg * MR + m;
+      const float v = even_plus_odd(acc[i][m]);
+      float sum = __shfl_sync(0xffffffffu, v, 0, kQuarters);
+#pragma unroll
+      for (int p = 1; p < kQuarters; ++p) sum += __shfl_sync(0xffffffffu, v, p, kQuarters);
+      if (q == m % kQuarters && n < N && row < M) y[static_cast<size_t>(row) * ldy + n] = sum;
     }
   }
 }
 
-template <typename TA, typename TW, typename TC>
-int launch(const void* x, const void* w, void* y, int M, int N, int K, int ldx, int ldy,
-           cudaStream_t stream) {
-  dim3 grid((N + kTN - 1) / kTN, (M + kTM - 1) / kTM);
-  launch_kernel(gemm_tn_simt_kernel<TA, TW, TC>, dim3(grid), dim3(256), 0, stream, 
-      static_cast<const TA*>(x), static_cast<const TW*>(w), static_cast<TC*>(y), M, N, K, ldx, ldy);
+// ---------------------------------------------------------------- many rows, and every other mix of types
+//
+// A block computes 64 x 64 outputs; its four groups of 64 threads take a quarter of K each, 8 x 8 outputs a thread.
+// Shared memory holds rows as they are (16 k of a row, 20 floats apart: conflict-free 16-byte reads along k, and
+// the pairs of a packed fma lie side by side).  The quarters meet in shared memory at the end.  kAsync: float
+// operands on 16-byte boundaries, copied through a ring of four stages; otherwise loads entry by entry.
+// Bound: the FFMA pipe and the shared-memory reads, one after the other (2,048 cycles each a stage; 31 of 74 TFLOP/s).
+// Plain instead of packed multiply-adds, or 8 x 4 outputs a thread on twice the warps, come out the same.
+constexpr int kTile = 64, kTlK = 16, kTlPitch = kTlK + 4, kTlStages = 4;
+constexpr int kTlN = 8;                                                 // outputs of a thread: 8 rows of x, kTlN of the weights
+constexpr int kTlCols = kTile / kTlN, kTlGroup = 8 * kTlCols, kTlThreads = kQuarters * kTlGroup;
+constexpr int kTlGroupFloats = 2 * kTile * kTlPitch;                     // x rows, then weight rows
+constexpr int kTlStageFloats = kQuarters * kTlGroupFloats;
+constexpr int kTlSmem = kTlStages * kTlStageFloats * 4;
+static_assert(kTlStages * kTlStageFloats >= (kQuarters - 1) * kTile * kTile, "the quarters' sums fit the ring");
+
+template <typename TA, typename TW, typename TC, bool kAsync>
+__global__ void __launch_bounds__(kTlThreads, 1)
+simt_tile_kernel(const TA* x, const TW* __restrict__ w, TC* y, int M, int N, int K, int ldx, int ldy) {
+  pdl_launch();
+  pdl_wait();
+  extern __shared__ __align__(16) float sm[];
+  const int m0 = blockIdx.y * kTile, n0 = blockIdx.x * kTile;
+  const int g = threadIdx.x / kTlGroup, t = threadIdx.x % kTlGroup;     // the quarter; the thread in its group
+  const int ty = t % 8, tx = t / 8;
+  const int ql = quarter_len(K);
+  const int steps = (ql + kTlK - 1) / kTlK;
+
+  auto ask = [&](int s) {
+    float* st = sm + (s % kTlStages) * kTlStageFloats + g * kTlGroupFloats;
+    if constexpr (kAsync) {
+#pragma unroll
+      for (int j = 0; j < 2 * kTile * 4 / kTlGroup; ++j) {
+        const int c = j * kTlGroup + t, row = c >> 2, piece = c & 3;           // rows 0..63 of x, then of the weights
+        const int off = s * kTlK + piece * 4, k = g * ql + off;
+        const bool is_x = j < kTile * 4 / kTlGroup;
+        const int r = is_x ? m0 + row : n0 + row - kTile;
+        const bool in = r < (is_x ? M : N) && off < ql && k < K;
+        const void* src = is_x ? static_cast<const void*>(x + static_cast<size_t>(r) * ldx + k)
+                               : static_cast<const void*>(w + static_cast<size_t>(r) * K + k);
+        copy16(st + row * kTlPitch + piece * 4, in ? src : static_cast<const void*>(w), in);
+      }
+    } else {
+      for (int c = t; c < 2 * kTile * kTlK; c += kTlGroup) {
+        const int row = c / kTlK, off = s * kTlK + c % kTlK, k = g * ql + off;
+        const bool is_x = row < kTile;
+        const int r = is_x ? m0 + row : n0 + row - kTile;
+        float v = 0.f;
+        if (r < (is_x ? M : N) && off < ql && k < K)
+          v = is_x ? to_float(x[static_cast<size_t>(r) * ldx + k]) : to_float(w[static_cast<size_t>(r) * K + k]);
+        st[row * kTlPitch + c % kTlK] = v;
+      }
+    }
+  };
+#pragma unroll
+  for (int s = 0; s < kTlStages - 1; ++s) {
+    if (s < steps) ask(s);
+    commit();
+  }
+  unsigned long long acc[8][kTlN];
+#pragma unroll
+  for (int i = 0; i < 8; ++i)
+#pragma unroll
+    for (int j = 0; j < kTlN; ++j) acc[i][j] = 0ull;
+
+  for (int s = 0; s < steps; ++s) {
+    wait_group<kTlStages - 2>();
+    __syncthreads();
+    if (s + kTlStages - 1 < steps) ask(s + kTlStages - 1);
+    commit();
+    const float* st = sm + (s % kTlStages) * kTlStageFloats + g * kTlGroupFloats;
+#pragma unroll
+    for (int p = 0; p < kTlK / 4; ++p) {
+      ulonglong2 a[8];
+#pragma unroll
+      for (int i = 0; i < 8; ++i) a[i] = *reinterpret_cast<const ulonglong2*>(st + (i * 8 + ty) * kTlPitch + p * 4);
+#pragma unroll
+      for (int j = 0; j < kTlN; ++j) {
+        const ulonglong2 b = *reinterpret_cast<const ulonglong2*>(st + (kTile + j * kTlCols + tx) * kTlPitch + p * 4);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) fma2(acc[i][j], a[i].x, b.x);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) fma2(acc[i][j], a[i].y, b.y);
+      }
+    }
+  }
+  wait_group<0>();
+  __syncthreads();                                   // the ring is free: the quarters' sums move in
+  if (g > 0) {
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+#pragma unroll
+      for (int j = 0; j < kTlN; ++j) sm[((g - 1) * kTile + i * 8 + ty) * kTile + j * kTlCols + tx] = even_plus_odd(acc[i][j]);
+  }
+  __syncthreads();
+  if (g > 0) return;
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    const int m = m0 + i * 8 + ty;
+#pragma unroll
+    for (int j = 0; j < kTlN; ++j) {
+      const int n = n0 + j * kTlCols + tx;
+      float sum = even_plus_odd(acc[i][j]);
+#pragma unroll
+      for (int q = 1; q < kQuarters; ++q) sum += sm[((q - 1) * kTile + i * 8 + ty) * kTile + j * kTlCols + tx];
+      if (m < M && n < N) y[static_cast<size_t>(m) * ldy + n] = from_float<TC>(sum);
+    }
+  }
+}
+
+template <auto kKernel>
+int raise_smem(int bytes) {
+  static std::atomic<bool> raised[64];                 // per device
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e == cudaSuccess && (dev >= 64 || !raised[dev].load(std::memory_order_relaxed))) {
+    e = cudaFuncSetAttribute(kKernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    if (e == cudaSuccess && dev < 64) raised[dev].store(true, std::memory_order_relaxed);
+  }
+  return static_cast<int>(e);
+}
+
+template <typename TA, typename TW, typename TC, bool kAsync>
+int launch_tile(const void* x, const void* w, void* y, int M, int N, int K, int ldx, int ldy, cudaStream_t stream) {
+  if (const int e = raise_smem<simt_tile_kernel<TA, TW, TC, kAsync>>(kTlSmem)) return e;
+  dim3 grid((N + kTile - 1) / kTile, (M + kTile - 1) / kTile);
+  launch_kernel(simt_tile_kernel<TA, TW, TC, kAsync>, grid, dim3(kTlThreads), kTlSmem, stream, static_cast<const TA*>(x),
+                static_cast<const TW*>(w), static_cast<TC*>(y), M, N, K, ldx, ldy);
   return static_cast<int>(cudaGetLastError());
+}
+
+template <int MR, int NPT, int MG, int STAGES>
+int launch_few(const float* x, const float* w, float* y, int M, int N, int K, int ldx, int ldy, cudaStream_t stream) {
+  constexpr int smem = STAGES * (16 * NPT + MR * MG) * kQuarters * kSkPitch * 4;
+  if (const int e = raise_smem<simt_few_kernel<MR, NPT, MG, STAGES>>(smem)) return e;
+  dim3 grid((N + 16 * NPT - 1) / (16 * NPT), (M + MR * MG - 1) / (MR * MG));
+  launch_kernel(simt_few_kernel<MR, NPT, MG, STAGES>, grid, dim3(64 * MG), smem, stream, w, x, y, M, N, K, ldx, ldy);
+  return static_cast<int>(cudaGetLastError());
+}
+
+// Up to 16 rows the weights' bytes bound the product: the kernel for few rows.  Above, that kernel (16 rows at a
+// time, 57 multiply-adds a clock and SM by its shared-memory reads on every SM) is the faster one while the tiles of
+// the other (96 or so a clock on as many SMs as it has tiles) leave a third of the chip without work.
+bool few_rows(int M, int N) {
+  const long long tiles = static_cast<long long>((M + kTile - 1) / kTile) * ((N + kTile - 1) / kTile);
+  return M <= 16 || tiles < 96;
+}
+
+int launch_f32(const void* xv, const void* wv, void* yv, int M, int N, int K, int ldx, int ldy, cudaStream_t stream) {
+  const bool aligned = K % 4 == 0 && ldx % 4 == 0 && reinterpret_cast<uintptr_t>(xv) % 16 == 0 &&
+                       reinterpret_cast<uintptr_t>(wv) % 16 == 0;
+  if (!aligned) return launch_tile<float, float, float, false>(xv, wv, yv, M, N, K, ldx, ldy, stream);
+  const long long chunks = (static_cast<long long>(M) + 15) / 16;
+  if (!few_rows(M, N) || chunks > 65535) return launch_tile<float, float, float, true>(xv, wv, yv, M, N, K, ldx, ldy, stream);
+  const float *x = static_cast<const float*>(xv), *w = static_cast<const float*>(wv);
+  float* y = static_cast<float*>(yv);
+  if (M == 1) return launch_few<1, 1, 1, 6>(x, w, y, M, N, K, ldx, ldy, stream);
+  if (M == 2) return launch_few<2, 1, 1, 6>(x, w, y, M, N, K, ldx, ldy, stream);
+  if (M <= 4) return launch_few<2, 1, 2, 6>(x, w, y, M, N, K, ldx, ldy, stream);
+  if (M <= 8) return launch_few<4, 1, 2, 5>(x, w, y, M, N, K, ldx, ldy, stream);
+  return launch_few<4, 2, 4, 4>(x, w, y, M, N, K, ldx, ldy, stream);
 }
 
 }  // namespace rl
@@ -85,14 +331,14 @@ int rl_gemm_tn_simt(const void* x, int x_dtype, const void* w, int w_dtype, void
   if (M <= 0 || N <= 0) return 0;
   const int code = x_dtype * 4 + w_dtype * 2 + y_dtype;
   switch (code) {
-    case 0: return launch<float, float, float>(x, w, y, M, N, K, ldx, ldy, stream);
-    case 1: return launch<float, float, bf16>(x, w, y, M, N, K, ldx, ldy, stream);
-    case 2: return launch<float, bf16, float>(x, w, y, M, N, K, ldx, ldy, stream);
-    case 3: return launch<float, bf16, bf16>(x, w, y, M, N, K, ldx, ldy, stream);
-    case 4: return launch<bf16, float, float>(x, w, y, M, N, K, ldx, ldy, stream);
-    case 5: return launch<bf16, float, bf16>(x, w, y, M, N, K, ldx, ldy, stream);
-    case 6: return launch<bf16, bf16, float>(x, w, y, M, N, K, ldx, ldy, stream);
-    case 7: return launch<bf16, bf16, bf16>(x, w, y, M, N, K, ldx, ldy, stream);
+    case 0: return launch_f32(x, w, y, M, N, K, ldx, ldy, stream);
+    case 1: return launch_tile<float, float, bf16, false>(x, w, y, M, N, K, ldx, ldy, stream);
+    case 2: return launch_tile<float, bf16, float, false>(x, w, y, M, N, K, ldx, ldy, stream);
+    case 3: return launch_tile<float, bf16, bf16, false>(x, w, y, M, N, K, ldx, ldy, stream);
+    case 4: return launch_tile<bf16, float, float, false>(x, w, y, M, N, K, ldx, ldy, stream);
+    case 5: return launch_tile<bf16, float, bf16, false>(x, w, y, M, N, K, ldx, ldy, stream);
+    case 6: return launch_tile<bf16, bf16, float, false>(x, w, y, M, N, K, ldx, ldy, stream);
+    case 7: return launch_tile<bf16, bf16, bf16, false>(x, w, y, M, N, K, ldx, ldy, stream);
   }
   return static_cast<int>(cudaErrorInvalidValue);
 }

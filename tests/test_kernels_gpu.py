@@ -92,6 +92,27 @@ def test_gemm_simt(tx, tw, ty, M, N, K):
         assert torch.equal(y1[0], y[M // 2])
 
 
+@pytest.mark.parametrize("N,K,ldx", [(16, 4, 4), (33, 36, 36), (70, 132, 140), (48, 516, 516), (2048, 260, 260), (40, 131, 131)])
+def test_gemm_simt_one_order_of_sums(N, K, ldx):
+    """Every kernel and row count (1, 2, up to 4, 8 and 16 rows in one block, several blocks, tiles of 64; K whose
+    quarters are ragged, empty or no multiple of a stage, and one that is not a multiple of four) gives a row the
+    same bits: those of four chains of even and odd k, restated in float64 to within float32 sums."""
+    full = torch.randn(200, ldx, device=DEV)
+    w = torch.randn(N, K, device=DEV)
+    ref = full[:, :K].double() @ w.double().T
+    rows = None
+    for M in (1, 2, 3, 4, 5, 8, 9, 16, 17, 33, 64, 65, 200):
+        y = torch.full((M, N + 3), 7.0, device=DEV)
+        kernels.gemm_tn_simt(full[:M, :K], w, y[:, :N])
+        assert torch.all(y[:, N:] == 7.0)
+        close(y[:, :N], ref[:M], 2e-6)
+        rows = y[:1, :N].clone() if rows is None else rows
+        assert torch.equal(y[:1, :N], rows), M
+        last = torch.empty(1, N, device=DEV)
+        kernels.gemm_tn_simt(full[M - 1:M, :K], w, last)
+        assert torch.equal(last, y[M - 1:M, :N]), M
+
+
 @pytest.mark.parametrize("M,N,K", [(1, 3072, 2048), (8, 1000, 384), (200, 704, 256), (64, 331, 200)])
 def test_linear_bfloat16(M, N, K):
     x = torch.randn(M, K, device=DEV).to(torch.bfloat16)
