@@ -20,6 +20,7 @@
 // reference's (src/cuda/kernels/common.cuh:105-140), as they must be for a seed to draw the
 // same token in both engines.  The fixed-point mass in integer atomics, the two-stage arg max
 // over chunks of a row and the kernels' organisation are this file's.
+#include <atomic>
 #include <cfloat>
 
 #include "common.cuh"
@@ -224,6 +225,33 @@ sample_partial_kernel(const float* __restrict__ logits, int vocab, int ld, Chunk
   if (threadIdx.x == 0) stats[row * kSampleChunks + chunk] = ChunkStat{b.v, b.i, s, 0.f};
 }
 
+// Greedy row with first-stage statistics, by one warp: combine the pieces (smaller index wins ties).
+__device__ __forceinline__ void greedy_from_stats(const float* l, const ChunkStat* stats, int row,
+                                                  int32_t* out_token, float* out_logprob) {
+  Best b{-FLT_MAX, 0x7fffffff};
+  for (int c = threadIdx.x; c < kSampleChunks; c += 32) {
+    const ChunkStat st = stats[c];
+    if (st.idx != 0x7fffffff) b = better(b, Best{st.mx, st.idx});
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    Best y;
+    y.v = __shfl_xor_sync(0xffffffffu, b.v, o);
+    y.i = __shfl_xor_sync(0xffffffffu, b.i, o);
+    b = better(b, y);
+  }
+  float sum = 0.f;
+  for (int c = threadIdx.x; c < kSampleChunks; c += 32) {
+    const ChunkStat st = stats[c];
+    if (st.idx != 0x7fffffff) sum += st.sumexp * expf(st.mx - b.v);
+  }
+  sum = warp_sum(sum);
+  if (threadIdx.x == 0) {
+    out_token[row] = b.i;
+    if (out_logprob) out_logprob[row] = l[b.i] - (b.v + logf(sum));
+  }
+}
+
 __global__ void __launch_bounds__(kSampleThreads)
 sample_kernel(const float* __restrict__ logits, int vocab, int ld, const float* __restrict__ temperature,
               const int32_t* __restrict__ top_k, const float* __restrict__ top_p,
@@ -236,31 +264,7 @@ sample_kernel(const float* __restrict__ logits, int vocab, int ld, const float* 
   const int row = blockIdx.x;
   const float* l = logits + static_cast<size_t>(row) * ld;
   if (stats != nullptr && temperature[row] <= 0.f) {
-    // greedy row with first-stage statistics: combine the pieces (smaller index wins ties)
-    if (threadIdx.x < 32) {
-      Best b{-FLT_MAX, 0x7fffffff};
-      for (int c = threadIdx.x; c < kSampleChunks; c += 32) {
-        const ChunkStat st = stats[row * kSampleChunks + c];
-        if (st.idx != 0x7fffffff) b = better(b, Best{st.mx, st.idx});
-      }
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) {
-        Best y;
-        y.v = __shfl_xor_sync(0xffffffffu, b.v, o);
-        y.i = __shfl_xor_sync(0xffffffffu, b.i, o);
-        b = better(b, y);
-      }
-      float sum = 0.f;
-      for (int c = threadIdx.x; c < kSampleChunks; c += 32) {
-        const ChunkStat st = stats[row * kSampleChunks + c];
-        if (st.idx != 0x7fffffff) sum += st.sumexp * expf(st.mx - b.v);
-      }
-      sum = warp_sum(sum);
-      if (threadIdx.x == 0) {
-        out_token[row] = b.i;
-        if (out_logprob) out_logprob[row] = l[b.i] - (b.v + logf(sum));
-      }
-    }
+    if (threadIdx.x < 32) greedy_from_stats(l, stats + row * kSampleChunks, row, out_token, out_logprob);
     return;
   }
 
@@ -317,7 +321,240 @@ sample_kernel(const float* __restrict__ logits, int vocab, int ld, const float* 
   }
 }
 
-// out[r] = log_softmax(logits[r, :])[target[r]]   (sampling.cu:288-300)
+// ---------------------------------------------------------------- sampled rows of a large vocabulary
+//
+// The same draw with a cluster of kRowCtas CTAs per row, each with its share of the row in shared memory.  The draw
+// takes ten passes over the row (arg max, sum, mass, four radix passes each of top-k and top-p, Gumbel); one CTA that
+// read 513 KB for each of them from L2 took 344 us for rows of 128,256 logits (B200, 1 to 32 rows with top-p), this
+// one 47 us at 21 rows together with the wait for the kernel before it.  Every pass here runs over 64 KB in shared memory, and the CTAs' counts or masses meet through distributed shared memory.
+// All selections are over integers (counts, fixed-point mass) or maxima, so they are the same bits in any order: the
+// tokens are those of sample_kernel.  A greedy row costs its first CTA what it did before.
+constexpr int kRowCtas = 8, kRowThreads = 512;
+// Rows from here on: below, a pass of one CTA is as short as a meeting of eight.
+constexpr int kRowVocab = 8192;
+constexpr int kRowMaxBytes = 200 * 1024;
+
+struct RowSmem {
+  float fscratch[32];
+  Best bscratch[32];
+  Best best;                           // this CTA's answers, for the cluster
+  float fsum;
+  unsigned long long mass;
+  unsigned long long hist[2][256];     // this CTA's bins (two sets in turn: one is cleared while peers may read the other)
+  unsigned long long total[256];       // the cluster's
+  uint32_t prefix;
+  unsigned long long remaining;
+};
+
+__device__ __forceinline__ void cluster_meet() {
+  asm volatile("barrier.cluster.arrive.aligned;\nbarrier.cluster.wait.aligned;" ::: "memory");
+}
+__device__ __forceinline__ uint32_t cluster_rank() {
+  uint32_t r;
+  asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+  return r;
+}
+__device__ __forceinline__ uint32_t peer_address(const void* p, uint32_t rank) {
+  uint32_t a;
+  asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(static_cast<uint32_t>(__cvta_generic_to_shared(p))), "r"(rank));
+  return a;
+}
+__device__ __forceinline__ uint32_t peer_u32(const void* p, uint32_t rank) {
+  uint32_t v;
+  asm volatile("ld.shared::cluster.u32 %0, [%1];" : "=r"(v) : "r"(peer_address(p, rank)) : "memory");
+  return v;
+}
+__device__ __forceinline__ unsigned long long peer_u64(const void* p, uint32_t rank) {
+  unsigned long long v;
+  asm volatile("ld.shared::cluster.u64 %0, [%1];" : "=l"(v) : "r"(peer_address(p, rank)) : "memory");
+  return v;
+}
+
+// The best of every CTA's `b` (which all threads of the CTA have).  `slot` is free again after the next meeting.
+__device__ Best cluster_best(Best b, Best* slot) {
+  if (threadIdx.x == 0) *slot = b;
+  cluster_meet();
+  Best r{-FLT_MAX, 0x7fffffff};
+#pragma unroll
+  for (int c = 0; c < kRowCtas; ++c)
+    r = better(r, Best{__uint_as_float(peer_u32(&slot->v, c)), static_cast<int>(peer_u32(&slot->i, c))});
+  return r;
+}
+
+// One radix selection over the cluster's rows: `add(i)` says what value i of this CTA's share adds to its bin (0: not
+// counted).  Walks the bins from the top until `want` is reached.  kMass: bins without mass are passed over, and if
+// rounding left the target out of reach the lowest one with mass is taken and all that remains kept; otherwise the
+// lowest bin is taken unseen.
+template <bool kMass, typename Add>
+__device__ uint32_t cluster_select(const float* l, int count, unsigned long long want, Add add, RowSmem& sh) {
+  uint32_t prefix = 0, mask = 0;
+  int turn = 0;
+  for (int b = threadIdx.x; b < 256; b += blockDim.x) sh.hist[0][b] = 0ull;
+  __syncthreads();
+  for (int shift = 24; shift >= 0; shift -= 8, turn ^= 1) {
+    for (int i = threadIdx.x; i < count; i += blockDim.x) {
+      const uint32_t key = order_key(l[i]);
+      if ((key & mask) == prefix) {
+        const unsigned long long q = add(l[i], key);
+        if (q != 0ull) atomicAdd(&sh.hist[turn][(key >> shift) & 255u], q);
+      }
+    }
+    cluster_meet();
+    if (threadIdx.x < 256) {
+      unsigned long long t = 0;
+#pragma unroll
+      for (int c = 0; c < kRowCtas; ++c) t += peer_u64(&sh.hist[turn][threadIdx.x], c);
+      sh.total[threadIdx.x] = t;
+      sh.hist[turn ^ 1][threadIdx.x] = 0ull;       // (read by peers before this meeting only)
+    }
+    __syncthreads();
+    if (threadIdx.x < 32) {
+      // lane n has the bins 255 - 8 n .. 248 - 8 n, from the top
+      const int top = 255 - 8 * static_cast<int>(threadIdx.x);
+      unsigned long long own = 0;
+#pragma unroll
+      for (int j = 0; j < 8; ++j) own += sh.total[top - j];
+      unsigned long long upto = own;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const unsigned long long y = __shfl_up_sync(0xffffffffu, upto, o);
+        if (static_cast<int>(threadIdx.x) >= o) upto += y;
+      }
+      // (a mass of zero is wanted where rounding ended an earlier pass: the first bin with mass then)
+      const unsigned long long least = kMass && want == 0ull ? 1ull : want;
+      const unsigned reached = __ballot_sync(0xffffffffu, upto >= least);
+      const unsigned filled = __ballot_sync(0xffffffffu, own != 0ull);
+      if (reached != 0u) {
+        if (static_cast<int>(threadIdx.x) == __ffs(reached) - 1) {
+          unsigned long long above = upto - own;
+          int b = top;
+          for (; b > top - 7; --b) {
+            if (above + sh.total[b] >= least) break;
+            above += sh.total[b];
+          }
+          sh.prefix = prefix | (static_cast<uint32_t>(b) << shift);
+          sh.remaining = want > above ? want - above : 0ull;
+        }
+      } else if (kMass) {
+        if (filled == 0u ? threadIdx.x == 0 : static_cast<int>(threadIdx.x) == 31 - __clz(filled)) {
+          int b = top - 7;
+          while (b < top && sh.total[b] == 0ull) ++b;
+          sh.prefix = prefix | (static_cast<uint32_t>(filled == 0u ? 0 : b) << shift);
+          sh.remaining = 0ull;
+        }
+      } else if (threadIdx.x == 31) {
+        sh.prefix = prefix;
+        sh.remaining = want - (upto - sh.total[0]);
+      }
+    }
+    __syncthreads();
+    prefix = sh.prefix;
+    want = sh.remaining;
+    mask |= 255u << shift;
+  }
+  cluster_meet();                                  // (no peer reads these bins any more)
+  return prefix;
+}
+
+__global__ void __launch_bounds__(kRowThreads)
+sample_cluster_kernel(const float* __restrict__ logits, int vocab, int ld, const float* __restrict__ temperature,
+                      const int32_t* __restrict__ top_k, const float* __restrict__ top_p,
+                      const uint32_t* __restrict__ seed_lo, const uint32_t* __restrict__ seed_hi,
+                      const int32_t* __restrict__ position, uint32_t stream_id, int32_t* __restrict__ out_token,
+                      float* __restrict__ out_logprob, const ChunkStat* __restrict__ stats) {
+  pdl_launch();
+  pdl_wait();
+  __shared__ RowSmem sh;
+  extern __shared__ __align__(16) float share[];
+  const int row = blockIdx.x / kRowCtas;
+  const uint32_t rank = cluster_rank();
+  const float* l = logits + static_cast<size_t>(row) * ld;
+  const float temp = temperature[row];
+  if (stats != nullptr && temp <= 0.f) {           // (the same for every CTA of the cluster)
+    if (rank == 0 && threadIdx.x < 32) greedy_from_stats(l, stats + row * kSampleChunks, row, out_token, out_logprob);
+    return;
+  }
+  const int per = ((vocab + kRowCtas - 1) / kRowCtas + 3) & ~3;
+  const int lo = min(vocab, static_cast<int>(rank) * per), count = min(vocab - lo, per);
+  if ((ld & 3) == 0 && (reinterpret_cast<uintptr_t>(logits) & 15) == 0) {
+    for (int i = threadIdx.x * 4; i + 4 <= count; i += blockDim.x * 4)
+      *reinterpret_cast<float4*>(share + i) = *reinterpret_cast<const float4*>(l + lo + i);
+    for (int i = (count & ~3) + threadIdx.x; i < count; i += blockDim.x) share[i] = l[lo + i];
+  } else {
+    for (int i = threadIdx.x; i < count; i += blockDim.x) share[i] = l[lo + i];
+  }
+  __syncthreads();
+  Best b{-FLT_MAX, 0x7fffffff};
+  for (int i = threadIdx.x; i < count; i += blockDim.x) b = better(b, Best{share[i], lo + i});
+  b = cluster_best(block_best(b, sh.bscratch), &sh.best);
+  const float mx = b.v;
+  float s = 0.f;
+  for (int i = threadIdx.x; i < count; i += blockDim.x) s += expf(share[i] - mx);
+  s = block_sum(s, sh.fscratch);
+  if (threadIdx.x == 0) sh.fsum = s;
+  cluster_meet();
+  s = 0.f;
+#pragma unroll
+  for (int c = 0; c < kRowCtas; ++c) s += __uint_as_float(peer_u32(&sh.fsum, c));
+  const float lse = mx + logf(s);
+
+  int token = b.i;
+  if (temp > 0.f) {
+    const float inv_t = 1.f / temp;
+    uint32_t thr = 0;
+    const int k = top_k[row];
+    if (k > 0 && k < vocab)
+      thr = cluster_select<false>(share, count, static_cast<unsigned long long>(k),
+                                  [](float, uint32_t) { return 1ull; }, sh);
+    const float p = top_p[row];
+    if (p < 1.f) {
+      // total mass of what top-k kept, in the same fixed point
+      unsigned long long part = 0;
+      for (int i = threadIdx.x; i < count; i += blockDim.x) {
+        if (order_key(share[i]) >= thr)
+          part += static_cast<unsigned long long>(expf((share[i] - mx) * inv_t) * kMassScale);
+      }
+      if (threadIdx.x == 0) sh.mass = 0ull;
+      __syncthreads();
+      if (part != 0ull) atomicAdd(&sh.mass, part);
+      cluster_meet();
+      unsigned long long total = 0;
+#pragma unroll
+      for (int c = 0; c < kRowCtas; ++c) total += peer_u64(&sh.mass, c);
+      const unsigned long long target =
+          static_cast<unsigned long long>(static_cast<double>(p) * static_cast<double>(total));
+      const uint32_t floor_key = thr;
+      const uint32_t thr_p = cluster_select<true>(
+          share, count, target > 0 ? target : 1ull,
+          [=](float v, uint32_t key) {
+            return key >= floor_key ? static_cast<unsigned long long>(expf((v - mx) * inv_t) * kMassScale) : 0ull;
+          },
+          sh);
+      thr = max(thr, thr_p);
+    }
+    Best g{-FLT_MAX, 0x7fffffff};
+    const uint32_t slo = seed_lo[row], shi = seed_hi[row];
+    const uint32_t pos = static_cast<uint32_t>(position[row]);
+    for (int i = threadIdx.x; i < count; i += blockDim.x) {
+      if (order_key(share[i]) < thr) continue;
+      const float u = uniform_open01(slo, shi, pos, stream_id, static_cast<uint32_t>(lo + i));
+      g = better(g, Best{(share[i] - mx) * inv_t - logf(-logf(u)), lo + i});
+    }
+    cluster_meet();                                // (sh.best has been read by every CTA)
+    g = cluster_best(block_best(g, sh.bscratch), &sh.best);
+    if (g.i != 0x7fffffff) token = g.i;
+  }
+  if (rank == 0 && threadIdx.x == 0) {
+    out_token[row] = token;
+    if (out_logprob) out_logprob[row] = l[token] - lse;
+  }
+  cluster_meet();                                  // (no CTA ends while a peer may read its shared memory)
+}
+
+// out[r] = log_softmax(logits[r, :])[target[r]]   (sampling.cu:288-300); NaN for a target outside the row.
+// One pass: a thread keeps a running maximum and the sum scaled to it over eight values at a time, which are all on
+// their way together (bound by the rows' bytes: 400 rows of 128,256 logits in 53 us, 3.9 TB/s; two passes a value
+// at a time took 138 us for 64 rows).
 __global__ void __launch_bounds__(512)
 gather_logprob_kernel(const float* __restrict__ logits, int vocab, int ld,
                       const int32_t* __restrict__ target, float* __restrict__ out) {
@@ -325,13 +562,29 @@ gather_logprob_kernel(const float* __restrict__ logits, int vocab, int ld,
   pdl_wait();
   __shared__ float scratch[32];
   const float* l = logits + static_cast<size_t>(blockIdx.x) * ld;
-  float m = -FLT_MAX;
-  for (int i = threadIdx.x; i < vocab; i += blockDim.x) m = fmaxf(m, l[i]);
-  m = block_max(m, scratch);
-  float s = 0.f;
-  for (int i = threadIdx.x; i < vocab; i += blockDim.x) s += expf(l[i] - m);
-  s = block_sum(s, scratch);
-  if (threadIdx.x == 0) out[blockIdx.x] = l[target[blockIdx.x]] - (m + logf(s));
+  constexpr int kHeld = 8;
+  float m = -FLT_MAX, s = 0.f;
+  for (int base = 0; base < vocab; base += kHeld * 512) {
+    float v[kHeld];
+#pragma unroll
+    for (int j = 0; j < kHeld; ++j) {
+      const int i = base + j * 512 + threadIdx.x;
+      v[j] = i < vocab ? l[i] : -INFINITY;
+    }
+    float top = m;
+#pragma unroll
+    for (int j = 0; j < kHeld; ++j) top = fmaxf(top, v[j]);
+    s *= expf(m - top);
+#pragma unroll
+    for (int j = 0; j < kHeld; ++j) s += expf(v[j] - top);
+    m = top;
+  }
+  const float mx = block_max(m, scratch);
+  s = block_sum(s * expf(m - mx), scratch);
+  if (threadIdx.x == 0) {
+    const int t = target[blockIdx.x];
+    out[blockIdx.x] = t >= 0 && t < vocab ? l[t] - (mx + logf(s)) : NAN;
+  }
 }
 
 }  // namespace rl
@@ -359,6 +612,35 @@ int rl_sample(const float* logits, int rows, int vocab, int ld, const float* tem
                     stats, kSampleChunks);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return static_cast<int>(e);
+  }
+  const int share = (((vocab + kRowCtas - 1) / kRowCtas + 3) & ~3) * 4;
+  if (vocab >= kRowVocab && share <= kRowMaxBytes) {
+    static std::atomic<bool> raised[64];              // per device
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return static_cast<int>(e);
+    if (dev >= 64 || !raised[dev].load(std::memory_order_relaxed)) {
+      e = cudaFuncSetAttribute(sample_cluster_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kRowMaxBytes);
+      if (e != cudaSuccess) return static_cast<int>(e);
+      if (dev < 64) raised[dev].store(true, std::memory_order_relaxed);
+    }
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(rows * kRowCtas);
+    cfg.blockDim = dim3(kRowThreads);
+    cfg.dynamicSmemBytes = share;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = kRowCtas;
+    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = pdl_enabled() ? 2 : 1;
+    e = cudaLaunchKernelEx(&cfg, sample_cluster_kernel, logits, vocab, ld, temperature, top_k, top_p,
+                                             seed_lo, seed_hi, position, static_cast<uint32_t>(stream_id), out_token,
+                                             out_logprob, static_cast<const ChunkStat*>(stats));
+    return static_cast<int>(e != cudaSuccess ? e : cudaGetLastError());
   }
   launch_kernel(sample_kernel, dim3(rows), dim3(kSampleThreads), 0, stream, logits, vocab, ld, temperature, top_k, top_p,
                                                      seed_lo, seed_hi, position, stream_id, out_token,

@@ -101,6 +101,42 @@ def test_large_vocabulary_top_k_membership():
     assert tok_m[0] == tok_g[0] and tok_m[2] == tok_g[2] and tok_m[1] in top[1] and tok_m[3] in top[3]
 
 
+@pytest.mark.parametrize("V,ld", [(8192, 8192), (8203, 8203), (8203, 8208), (20001, 20004)])
+@pytest.mark.parametrize("T,k,p", [(1.0, 7, 1.0), (0.7, 0, 0.05), (1.3, 50, 0.6), (0.9, 1, 1.0), (2.0, 8191, 1e-6)])
+def test_draw_over_a_cluster_equals_the_plain_restatement(V, ld, T, k, p):
+    """Rows cut over a cluster of CTAs (large vocabularies): the last CTA's share is short or ragged, rows start off
+    16-byte boundaries, logits tie at the thresholds and across shares, others are -inf, one row is greedy."""
+    rng = np.random.RandomState(V + k)
+    l = (rng.randn(5, V) * 3).astype(np.float32)
+    l[1] = np.round(l[1])                                  # many ties at every threshold
+    l[2, rng.rand(V) < 0.9] = -np.inf
+    l[3, V - 1] = l[3, 0] = l[3].max() + 1.0               # the maximum twice, in the first and the last share
+    buf = torch.full((5, ld), float("nan"), device=DEV)
+    buf[:, :V] = torch.from_numpy(l).to(DEV)
+    temp = np.array([T, T, T, T, 0.0], dtype=np.float32)
+    tok, lp = run(buf[:, :V], temp, k, p, 1234567890123, np.arange(5) + 3)
+    for r in range(4):
+        assert tok[r] == P.gumbel_draw(l[r], T, k, p, 1234567890123, r + 3), r
+    assert tok[4] == int(l[4].argmax())
+    want = torch.log_softmax(torch.from_numpy(l).double(), -1)[torch.arange(5), torch.from_numpy(tok.astype(np.int64))]
+    assert np.abs(lp - want.numpy()).max() < 1e-4
+
+
+@pytest.mark.parametrize("V", [1, 511, 4096, 50001])
+def test_gather_logprob_one_pass(V):
+    """Rows shorter than a block's first loads, on its edge, and ragged; values far apart and -inf."""
+    l = torch.randn(3, V, device=DEV) * 30
+    if V > 1:
+        l[1, ::2] = -float("inf")
+    l[2] -= 1e4
+    tgt = torch.tensor([0, V // 2 | 1 if V > 1 else 0, V - 1], device=DEV, dtype=torch.int32).clamp(max=V - 1)
+    out = torch.empty(3, device=DEV)
+    kernels.gather_logprob(l, 3, tgt, out)
+    want = torch.log_softmax(l.double(), -1)[torch.arange(3), tgt.long()]
+    fine = torch.isfinite(want)          # (float32 sums of values about 1e4: a unit in the last place is 1e-3)
+    assert torch.equal(torch.isfinite(out), fine) and (out.double() - want)[fine].abs().max().item() < 2e-3
+
+
 def test_gather_logprob():
     l = torch.randn(9, 777, device=DEV) * 3
     tgt = torch.randint(0, 777, (9,), device=DEV, dtype=torch.int32)
