@@ -57,21 +57,30 @@ class Workspace:
 
     def __init__(self, device: torch.device):
         self.device = device
-        self._bufs: Dict[str, torch.Tensor] = {}
+        self._bufs: Dict[Tuple[str, torch.dtype], torch.Tensor] = {}
+        self._views: Dict[Tuple, torch.Tensor] = {}      # what was handed out: a step asks for the same ones again
         self._retired: List[torch.Tensor] = []
 
     def get(self, name: str, shape: Tuple[int, ...], dtype: torch.dtype) -> torch.Tensor:
+        view = self._views.get((name, shape, dtype))
+        if view is not None:
+            return view
         n = 1
         for s in shape:
             n *= int(s)
-        key = f"{name}:{dtype}"
+        key = (name, dtype)
         buf = self._bufs.get(key)
         if buf is None or buf.numel() < n:
             if buf is not None:
                 self._retired.append(buf)   # a captured graph may still point at it
             buf = torch.empty(max(n, 1), dtype=dtype, device=self.device)
             self._bufs[key] = buf
-        return buf[:n].view(shape)
+            for k in [k for k in self._views if k[0] == name and k[2] is dtype]:
+                del self._views[k]              # (views of the buffer that this one replaces)
+        view = buf[:n].view(shape)
+        if len(self._views) < 1024:             # (shapes are a part's widest: a model has some dozens of them)
+            self._views[(name, shape, dtype)] = view
+        return view
 
     def nbytes(self) -> int:
         return sum(b.numel() * b.element_size() for b in self._bufs.values())
