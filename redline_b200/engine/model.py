@@ -157,11 +157,11 @@ class DecoderModel:
         return sum(p.nbytes() for p in self._named_parts())
 
     # ------------------------------------------------------------- forward
-    def forward(self, ctx, caches, states, logits: torch.Tensor) -> torch.Tensor:
-        """Runs the step's tokens; returns logits[:R] (float32) at the wanted rows.
-        ``caches[i]`` / ``states[i]`` belong to run-order entry i (None where unused)."""
+    def body(self, ctx, caches, states) -> Tuple[torch.Tensor, Optional[torch.Tensor]]:
+        """Runs the step's tokens through every block; returns the stream's rows and what is still to be added to
+        them before the final norm (or None)."""
         rt = self.rt
-        T, R = ctx.T, ctx.R
+        T = ctx.T
         ws = rt.workspace
         residual = ws.get("residual", (rt.max_tokens, self.spec.hidden_size), torch.float32)[:T]
         self.embedding.forward(ctx, residual)
@@ -194,13 +194,29 @@ class DecoderModel:
             if self.nvtx_layers:
                 torch.cuda.nvtx.range_pop()
         ctx.block_hand = ctx.block_next_norm = ctx.block_normed = ctx.block_next = None
+        return residual, pending
+
+    def forward(self, ctx, caches, states, logits: torch.Tensor) -> torch.Tensor:
+        """Runs the step's tokens; returns logits[:R] (float32) at the wanted rows.
+        ``caches[i]`` / ``states[i]`` belong to run-order entry i (None where unused)."""
+        rt = self.rt
+        R = ctx.R
+        residual, pending = self.body(ctx, caches, states)
         head_w = getattr(self.head, "weight", None)
         if R > 0 and pending is None and self.head.forward_from(residual, self.final_norm, ctx.logit_rows, R, logits):
             op_mark(ctx, "final_norm+lm_head", head_w, R, nbytes=R * logits.shape[1] * 2.0)
         elif R > 0:
-            xr = ws.get("head.in", (logits.shape[0], self.spec.hidden_size), rt.dtype)[:R]
+            xr = rt.workspace.get("head.in", (logits.shape[0], self.spec.hidden_size), rt.dtype)[:R]
             self.final_norm.add_norm(residual, pending, xr, rows_idx=ctx.logit_rows, rows=R)
             op_mark(ctx, "final_norm", nbytes=R * self.spec.hidden_size * 6.0)
             self.head.forward(xr, R, logits)
             op_mark(ctx, "lm_head", head_w, R, nbytes=R * logits.shape[1] * 2.0)     # (the logits are float32: 2 more bytes each)
         return logits[:R]
+
+    def head_over(self, residual: torch.Tensor, pending: Optional[torch.Tensor], logits: torch.Tensor) -> torch.Tensor:
+        """Logits of every row that ``body`` left in ``residual`` / ``pending`` (at most as many as ``logits`` has)."""
+        rows = residual.shape[0]
+        xr = self.rt.workspace.get("head.rows", (logits.shape[0], self.spec.hidden_size), self.rt.dtype)[:rows]
+        self.final_norm.add_norm(residual, pending, xr, rows=rows)
+        self.head.forward(xr, rows, logits)
+        return logits[:rows]

@@ -171,6 +171,21 @@ class ModelRunner:
                 self.profiler.end()
         return self.logits[:ctx.R], ctx
 
+    def run_body(self, segments: Sequence[Segment]) -> Tuple[torch.Tensor, Optional[torch.Tensor]]:
+        """Runs the segments' tokens (none of which wants its logits) and returns what ``DecoderModel.body`` does:
+        for callers that take the logits of more rows than the logits buffer has, block by block (``score``)."""
+        ctx = self.builder.build(segments)
+        if self.profiler is not None:
+            ctx.profiler = self.profiler
+            self.profiler.begin("prefill")
+        before = kernels.LAUNCHES
+        out = self.model.body(ctx, self._caches, self._states)
+        self.num_eager_steps += 1
+        self.num_kernel_launches += kernels.LAUNCHES - before
+        if self.profiler is not None:
+            self.profiler.end()
+        return out
+
     def _forward(self, ctx: StepContext, sample: bool, resolve: bool) -> None:
         if resolve:
             kernels.resolve_ids(ctx.token_ids, ctx.token_src, self.sampler.tokens, ctx.T)
