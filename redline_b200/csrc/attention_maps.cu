@@ -114,12 +114,34 @@ struct MapsDecodeArgs {
   TailArgs<T> tail;
 };
 
+// A piece of a row as it lies in memory: 16 bytes, or one element where rows do not divide into those.
+template <typename T, int E>
+struct Piece {
+  uint4 v;
+  __device__ __forceinline__ void load(const T* p) { v = *reinterpret_cast<const uint4*>(p); }
+  __device__ __forceinline__ void zero() { v = make_uint4(0, 0, 0, 0); }
+  __device__ __forceinline__ void get(float* f) const { load16(reinterpret_cast<const T*>(&v), f); }
+};
+template <typename T>
+struct Piece<T, 1> {
+  T v;
+  __device__ __forceinline__ void load(const T* p) { v = *p; }
+  __device__ __forceinline__ void zero() { v = from_float<T>(0.f); }
+  __device__ __forceinline__ void get(float* f) const { f[0] = to_float(v); }
+};
+
 // Lane l of the 8 that share a key takes elements l, l + 8, ... of the key in pieces of E elements.
+//
+// A launch is a few keys to each SM (eight sequences of 540 keys, 4 kv heads: 160 CTAs with 64 KB each), so what
+// bounds it is the chain of round trips to memory, not bytes.  A thread therefore asks for all its pieces of the partition's
+// keys AND values before it multiplies any (16 pieces of each where rows have 128 entries or less in 16 bits; longer rows
+// in batches), and reads the work item and its pages while the kernel before still runs.  Decode steps of eight such
+// sequences, with the merge below: 0.52 -> 0.48 ms (two layers of 64 / 128 entries and two maps), 0.36 -> 0.31 ms (three of
+// 128 / 128 and 96 entries).
 template <typename T>
 __global__ void __launch_bounds__(kThreads)
 maps_decode_kernel(const MapsDecodeArgs<T> a) {
   pdl_launch();
-  pdl_wait();
   constexpr int VEC = Vec16<T>::N;
   constexpr int E = (kD % VEC == 0) ? VEC : 1;          // piece of a key
   constexpr int CH = kD / E;
@@ -127,7 +149,12 @@ maps_decode_kernel(const MapsDecodeArgs<T> a) {
   constexpr int EVV = (kDV % VEC == 0 && kVS % VEC == 0) ? VEC : 1;         // piece of a value row
   constexpr int CHV = kDV / EVV;
   constexpr int CPLV = (CHV + kLPK - 1) / kLPK;
-  __shared__ float qs[kRows][kD];
+  constexpr int IT = kPart / kKeysPerIter;               // keys of a thread
+  constexpr int KB = CPL <= 2 ? IT : (CPL <= 4 ? 4 : (CPL <= 8 ? 2 : 1));                // ... asked for at once
+  constexpr int VB = CPLV <= 2 ? IT : (CPLV <= 4 ? 4 : (CPLV <= 8 ? 2 : 1));                 // ... values
+  constexpr bool kValuesAhead = VB == IT;                // the partition's values are asked for with its keys
+  static_assert(IT % KB == 0 && IT % VB == 0, "whole batches");
+  __shared__ __align__(16) float qs[kM][kRows][kD];
   __shared__ float sc[kRows][kPart];
   __shared__ float red[kThreads / 32][kRows][kDV];
   __shared__ float stat_m[kRows], stat_l[kRows];
@@ -136,58 +163,92 @@ maps_decode_kernel(const MapsDecodeArgs<T> a) {
   const int G = a.heads / a.kv_heads;
   const int groups = (G + kRows - 1) / kRows;
   const int part = blockIdx.x, kvh = blockIdx.y / groups, g0 = (blockIdx.y % groups) * kRows, item = blockIdx.z;
+  // (items and block tables were written before the step's kernels began)
   const int4 info = a.items[item];
   const int tok = info.x, seq = info.y, ctx = info.z;
   const int me = ctx - 1;                                // the query's position
   const int base = part * kPart;
   const int j_hi = min(ctx, base + kPart);
   const int first = first_key(me, a.mask);
-  if (!range_visible(base, j_hi, me, first, a.mask)) return;
+  if (!range_visible(base, j_hi, me, first, a.mask)) {
+    pdl_wait();       // (no grid completes before the one before it)
+    return;
+  }
   const int lane8 = threadIdx.x % kLPK, slot = threadIdx.x / kLPK;
   const int warp = threadIdx.x >> 5;
   const int32_t* bt = a.block_table + static_cast<size_t>(seq) * a.max_blocks;
   const float inv_cap = a.softcap > 0.f ? 1.f / a.softcap : 0.f;
-  // the pages of this thread's keys (key base + it * 16 + slot), read once
-  int pages[kPart / kKeysPerIter];
+  const int ng = min(kRows, G - g0);
+  // this thread's keys (key base + it * 16 + slot): whether they are visible, and their pages
+  int pages[IT];
+  unsigned live = 0;
 #pragma unroll
-  for (int it = 0; it < kPart / kKeysPerIter; ++it) {
+  for (int it = 0; it < IT; ++it) {
     const int j = base + it * kKeysPerIter + slot;
-    pages[it] = (j < j_hi && key_visible(j, me, first, a.mask)) ? bt[j / a.page_size] : 0;
+    const bool ok = j < j_hi && key_visible(j, me, first, a.mask);
+    live |= ok ? 1u << it : 0u;
+    pages[it] = ok ? bt[j / a.page_size] : 0;
   }
+  pdl_wait();         // q and the newest keys and values come from the kernels before this one
+
+  Piece<T, E> kr[KB][CPL];
+  auto ask_keys = [&](int m, int it0) {
+#pragma unroll
+    for (int b = 0; b < KB; ++b) {
+      const int it = it0 + b, j = base + it * kKeysPerIter + slot;
+      const T* kp = a.kcache + ((static_cast<size_t>(pages[it]) * (a.kv_heads * kM) + kvh * kM + m) * a.page_size + j % a.page_size) * kD;
+#pragma unroll
+      for (int c = 0; c < CPL; ++c) {
+        const int ch = lane8 + c * kLPK;
+        if ((live >> it & 1) && ch < CH) kr[b][c].load(kp + ch * E);
+        else kr[b][c].zero();
+      }
+    }
+  };
+  Piece<T, EVV> vr[VB][CPLV];
+  auto ask_values = [&](int it0) {
+#pragma unroll
+    for (int b = 0; b < VB; ++b) {
+      const int it = it0 + b, j = base + it * kKeysPerIter + slot;
+      const T* vp = a.vcache + ((static_cast<size_t>(pages[it]) * a.kv_heads + kvh) * a.page_size + j % a.page_size) * kVS;
+#pragma unroll
+      for (int c = 0; c < CPLV; ++c) {
+        const int ch = lane8 + c * kLPK;
+        if ((live >> it & 1) && ch < CHV) vr[b][c].load(vp + ch * EVV);
+        else vr[b][c].zero();
+      }
+    }
+  };
+  ask_keys(0, 0);
+  for (int i = threadIdx.x; i < kM * kRows * kD; i += kThreads) {
+    const int m = i / (kRows * kD), g = (i - m * (kRows * kD)) / kD, d = i % kD;
+    qs[m][g][d] = g < ng ? to_float(a.q[static_cast<size_t>(tok) * a.q_stride + ((kvh * G + g0 + g) * kM + m) * kD + d]) * a.scale
+                         : 0.f;
+  }
+  if (kValuesAhead) ask_values(0);
+  __syncthreads();
 
   for (int m = 0; m < kM; ++m) {
-    const int khead = kvh * kM + m;
-    {
-      const int ng = min(kRows, G - g0);
-      __syncthreads();
-      for (int i = threadIdx.x; i < kRows * kD; i += kThreads) {
-        const int g = i / kD, d = i - g * kD;
-        qs[g][d] = g < ng ? to_float(a.q[static_cast<size_t>(tok) * a.q_stride +
-                                         ((kvh * G + g0 + g) * kM + m) * kD + d]) * a.scale
-                          : 0.f;
-      }
-      __syncthreads();
-      // ---- scores (every lane of a warp makes the same number of trips: the shuffles need all of them)
+    // ---- scores (every lane of a warp makes the same number of trips: the shuffles need all of them)
 #pragma unroll
-      for (int it = 0; it < kPart / kKeysPerIter; ++it) {
-        const int j = base + it * kKeysPerIter + slot;
-        const bool live = j < j_hi && key_visible(j, me, first, a.mask);
-        const size_t page = live ? pages[it] : 0;
-        const T* kp = a.kcache + ((page * (a.kv_heads * kM) + khead) * a.page_size + j % a.page_size) * kD;
+    for (int it0 = 0; it0 < IT; it0 += KB) {
+      if (KB < IT && (m > 0 || it0 > 0)) ask_keys(m, it0);
+#pragma unroll
+      for (int b = 0; b < KB; ++b) {
+        const int it = it0 + b, j = base + it * kKeysPerIter + slot;
         float dot[kRows];
 #pragma unroll
         for (int g = 0; g < kRows; ++g) dot[g] = 0.f;
 #pragma unroll
         for (int c = 0; c < CPL; ++c) {
           const int ch = lane8 + c * kLPK;
-          if (live && ch < CH) {
+          if (CH % kLPK == 0 || ch < CH) {
             float kf[E];
-            if (E == 1) kf[0] = to_float(kp[ch]);
-            else load16(kp + ch * E, kf);
+            kr[b][c].get(kf);
 #pragma unroll
             for (int g = 0; g < kRows; ++g) {
 #pragma unroll
-              for (int e = 0; e < E; ++e) dot[g] += kf[e] * qs[g][ch * E + e];
+              for (int e = 0; e < E; ++e) dot[g] += kf[e] * qs[m][g][ch * E + e];
             }
           }
         }
@@ -197,102 +258,112 @@ maps_decode_kernel(const MapsDecodeArgs<T> a) {
           v += __shfl_xor_sync(0xffffffffu, v, 1);
           v += __shfl_xor_sync(0xffffffffu, v, 2);
           v += __shfl_xor_sync(0xffffffffu, v, 4);
-          if (lane8 == 0 && j < j_hi) {
-            if (a.softcap > 0.f) v = a.softcap * tanhf(v * inv_cap);
-            if (a.tail.slopes != nullptr && g < ng) v -= a.tail.slopes[kvh * G + g0 + g] * static_cast<float>(me - j);
-            sc[g][j - base] = live ? v : -INFINITY;
-          }
+          if (lane8 == 0 && j < j_hi) sc[g][j - base] = v;
         }
       }
-      __syncthreads();
-      // ---- softmax statistics of this partition, one warp per row
-      for (int g = warp; g < ng; g += kThreads / 32) {
-        float mx = -INFINITY;
-        for (int j = base + (threadIdx.x & 31); j < j_hi; j += 32) mx = fmaxf(mx, sc[g][j - base]);
-        mx = warp_max(mx);
-        float l = 0.f;
-        for (int j = base + (threadIdx.x & 31); j < j_hi; j += 32) {
-          const float p = expf(sc[g][j - base] - mx);      // masked keys: exp(-inf) = 0
-          sc[g][j - base] = p;
-          l += p;
+    }
+    if (KB == IT && m + 1 < kM) ask_keys(m + 1, 0);
+    __syncthreads();
+    // ---- cap, slopes and softmax statistics of this partition, one warp per row, a lane per key and 32 more
+    for (int g = warp; g < ng; g += kThreads / 32) {
+      float x[kPart / 32];
+      float mx = -INFINITY;
+#pragma unroll
+      for (int k = 0; k < kPart / 32; ++k) {
+        const int j = base + k * 32 + (threadIdx.x & 31);
+        x[k] = -INFINITY;
+        if (j < j_hi && key_visible(j, me, first, a.mask)) {
+          float v = sc[g][j - base];
+          if (a.softcap > 0.f) v = a.softcap * tanhf(v * inv_cap);
+          if (a.tail.slopes != nullptr) v -= a.tail.slopes[kvh * G + g0 + g] * static_cast<float>(me - j);
+          x[k] = v;
         }
-        l = warp_sum(l);
-        if ((threadIdx.x & 31) == 0) {
-          stat_m[g] = mx;
-          stat_l[g] = l;
-        }
+        mx = fmaxf(mx, x[k]);
       }
-      __syncthreads();
-      // ---- P V
-      float acc[kRows][CPLV][EVV];
+      mx = warp_max(mx);
+      float l = 0.f;
 #pragma unroll
-      for (int g = 0; g < kRows; ++g)
+      for (int k = 0; k < kPart / 32; ++k) {
+        const float p = expf(x[k] - mx);                   // masked keys: exp(-inf) = 0
+        sc[g][k * 32 + (threadIdx.x & 31)] = p;
+        l += p;
+      }
+      l = warp_sum(l);
+      if ((threadIdx.x & 31) == 0) {
+        stat_m[g] = mx;
+        stat_l[g] = l;
+      }
+    }
+    __syncthreads();
+    // ---- P V
+    float acc[kRows][CPLV][EVV];
 #pragma unroll
-        for (int c = 0; c < CPLV; ++c)
+    for (int g = 0; g < kRows; ++g)
 #pragma unroll
-          for (int e = 0; e < EVV; ++e) acc[g][c][e] = 0.f;
+      for (int c = 0; c < CPLV; ++c)
 #pragma unroll
-      for (int it = 0; it < kPart / kKeysPerIter; ++it) {
-        const int j = base + it * kKeysPerIter + slot;
-        if (j >= j_hi || !key_visible(j, me, first, a.mask)) continue;
-        const size_t page = pages[it];
-        const T* vp = a.vcache + ((page * a.kv_heads + kvh) * a.page_size + j % a.page_size) * kVS;
+        for (int e = 0; e < EVV; ++e) acc[g][c][e] = 0.f;
+#pragma unroll
+    for (int it0 = 0; it0 < IT; it0 += VB) {
+      if (!kValuesAhead) ask_values(it0);
+#pragma unroll
+      for (int b = 0; b < VB; ++b) {
+        const int it = it0 + b;
+        if (!(live >> it & 1)) continue;                 // (its weight is zero, or its place in sc was never written)
         float p[kRows];
 #pragma unroll
-        for (int g = 0; g < kRows; ++g) p[g] = g < ng ? sc[g][j - base] : 0.f;
+        for (int g = 0; g < kRows; ++g) p[g] = g < ng ? sc[g][it * kKeysPerIter + slot] : 0.f;
+#pragma unroll
+        for (int c = 0; c < CPLV; ++c) {
+          float vf[EVV];
+          vr[b][c].get(vf);
+#pragma unroll
+          for (int g = 0; g < kRows; ++g)
+#pragma unroll
+            for (int e = 0; e < EVV; ++e) acc[g][c][e] += p[g] * vf[e];
+        }
+      }
+    }
+    // lanes 8 and 16 apart hold other keys of the same piece
+#pragma unroll
+    for (int g = 0; g < kRows; ++g)
+#pragma unroll
+      for (int c = 0; c < CPLV; ++c)
+#pragma unroll
+        for (int e = 0; e < EVV; ++e) {
+          float v = acc[g][c][e];
+          v += __shfl_xor_sync(0xffffffffu, v, 8);
+          v += __shfl_xor_sync(0xffffffffu, v, 16);
+          acc[g][c][e] = v;
+        }
+    if ((threadIdx.x & 31) < kLPK) {
+#pragma unroll
+      for (int g = 0; g < kRows; ++g)
 #pragma unroll
         for (int c = 0; c < CPLV; ++c) {
           const int ch = lane8 + c * kLPK;
           if (ch < CHV) {
-            float vf[EVV];
-            if (EVV == 1) vf[0] = to_float(vp[ch]);
-            else load16(vp + ch * EVV, vf);
 #pragma unroll
-            for (int g = 0; g < kRows; ++g)
-#pragma unroll
-              for (int e = 0; e < EVV; ++e) acc[g][c][e] += p[g] * vf[e];
+            for (int e = 0; e < EVV; ++e) red[warp][g][ch * EVV + e] = acc[g][c][e];
           }
         }
-      }
-      // lanes 8 and 16 apart hold other keys of the same piece
+    }
+    __syncthreads();
+    for (int i = threadIdx.x; i < ng * kDV; i += kThreads) {
+      const int g = i / kDV, d = i - g * kDV;
+      float v = 0.f;
 #pragma unroll
-      for (int g = 0; g < kRows; ++g)
-#pragma unroll
-        for (int c = 0; c < CPLV; ++c)
-#pragma unroll
-          for (int e = 0; e < EVV; ++e) {
-            float v = acc[g][c][e];
-            v += __shfl_xor_sync(0xffffffffu, v, 8);
-            v += __shfl_xor_sync(0xffffffffu, v, 16);
-            acc[g][c][e] = v;
-          }
-      if ((threadIdx.x & 31) < kLPK) {
-#pragma unroll
-        for (int g = 0; g < kRows; ++g)
-#pragma unroll
-          for (int c = 0; c < CPLV; ++c) {
-            const int ch = lane8 + c * kLPK;
-            if (ch < CHV) {
-#pragma unroll
-              for (int e = 0; e < EVV; ++e) red[warp][g][ch * EVV + e] = acc[g][c][e];
-            }
-          }
-      }
-      __syncthreads();
-      for (int i = threadIdx.x; i < ng * kDV; i += kThreads) {
-        const int g = i / kDV, d = i - g * kDV;
-        float v = 0.f;
-#pragma unroll
-        for (int w = 0; w < kThreads / 32; ++w) v += red[w][g][d];
-        const int qrow = (kvh * G + g0 + g) * kM + m;
-        const size_t row = (static_cast<size_t>(item) * (a.heads * kM) + qrow) * a.max_parts + part;
-        a.part_o[row * kDV + d] = v;
-        if (d == 0) {
-          a.part_ml[row * 2] = stat_m[g];
-          a.part_ml[row * 2 + 1] = stat_l[g];
-        }
+      for (int w = 0; w < kThreads / 32; ++w) v += red[w][g][d];
+      const int qrow = (kvh * G + g0 + g) * kM + m;
+      const size_t row = (static_cast<size_t>(item) * (a.heads * kM) + qrow) * a.max_parts + part;
+      a.part_o[row * kDV + d] = v;
+      if (d == 0) {
+        a.part_ml[row * 2] = stat_m[g];
+        a.part_ml[row * 2 + 1] = stat_l[g];
       }
     }
+    // (the next map's scores go into sc, which every thread has read; its statistics and sums are written
+    // behind the barriers after those scores)
   }
 }
 
@@ -315,19 +386,24 @@ maps_merge_kernel(const MapsDecodeArgs<T> a) {
   __syncthreads();
   for (int m = 0; m < kM; ++m) {
     const size_t row0 = (static_cast<size_t>(item) * (a.heads * kM) + head * kM + m) * a.max_parts;
+    auto visible = [&](int p) { return range_visible(p * kPart, min(ctx, (p + 1) * kPart), me, first, a.mask); };
     float mx = -INFINITY;
-    for (int p = p_lo; p <= p_hi; ++p)
-      if (range_visible(p * kPart, min(ctx, (p + 1) * kPart), me, first, a.mask)) mx = fmaxf(mx, a.part_ml[(row0 + p) * 2]);
+    for (int p = p_lo + static_cast<int>(threadIdx.x); p <= p_hi; p += kThreads)
+      if (visible(p)) mx = fmaxf(mx, a.part_ml[(row0 + p) * 2]);
+    mx = block_max(mx, scratch);
     const float coef = m == 0 ? 1.f : -a.lambda;
     const bool sunk = kM == 1 && a.tail.sink != nullptr;
     if (sunk) mx = fmaxf(mx, a.tail.sink[head]);
     for (int d = threadIdx.x; d < kDV; d += kThreads) {
       float num = 0.f, den = sunk ? expf(a.tail.sink[head] - mx) : 0.f;
-      for (int p = p_lo; p <= p_hi; ++p) {
-        if (!range_visible(p * kPart, min(ctx, (p + 1) * kPart), me, first, a.mask)) continue;
-        const float w = expf(a.part_ml[(row0 + p) * 2] - mx);
-        num += w * a.part_o[(row0 + p) * kDV + d];
-        den += w * a.part_ml[(row0 + p) * 2 + 1];
+#pragma unroll 4
+      for (int p = p_lo; p <= p_hi; ++p) {               // (loads without a branch around them: four partitions at once)
+        const bool ok = visible(p);
+        const float ml = ok ? a.part_ml[(row0 + p) * 2] : -INFINITY, dn = ok ? a.part_ml[(row0 + p) * 2 + 1] : 0.f;
+        const float po = ok ? a.part_o[(row0 + p) * kDV + d] : 0.f;
+        const float w = ok ? expf(ml - mx) : 0.f;
+        num += w * po;
+        den += w * dn;
       }
       o[d] += coef * (num / den);
     }
