@@ -7,10 +7,9 @@
 // one after another, longest first, and the pipeline runs on across items.  Per item the keys
 // come in tiles of 128; for each slot and key tile:
 //   S = Q K^T      tcgen05.mma, 128 x 128, k = head size, accumulator in tensor memory
-//   softmax        two threads per query row (eight warps per slot, so that every scheduler of the SM
-//                  has four row warps to choose from) read the row of S from tensor memory, each
-//                  keeps the running maximum of the row and the denominator of its 64 keys in
-//                  float32 and writes their P as bfloat16 back into tensor memory
+//   softmax        a thread per query row (four warps per slot) reads the row of S from tensor memory,
+//                  keeps its running maximum and denominator in float32 and writes P as bfloat16 back
+//                  into tensor memory
 //   O += P V       tcgen05.mma with P as the A operand from tensor memory and V as it lies in the
 //                  cache (a key's values contiguous: the B operand in MN-major form); O stays in
 //                  tensor memory for the whole item and is accumulated by the tensor core
@@ -27,10 +26,17 @@
 // into registers, so it is done before they have finished with this tile, and the rows never wait
 // for the tensor core.  At head size 128 the columns are all taken: P lies over the first 64
 // columns of its S, and the next S product has to wait for the O product that reads P.
-// Warp roles: warps 0-7 rows of slot 0, warps 8-15 rows of slot 1 (warp w owns TMEM lanes
-// 32 (w % 4) ..), warp 16 brings both Q tiles once per item and the K tiles, warp 17 the V tiles,
+// What bounds it is the row threads: per 128 x 128 tile and slot 2,048 cycles of the special-function unit for both
+// slots' exponentials, of 3,700 that a pair of tiles takes, the rest their other instructions and the hand-overs.  One
+// thread to a row takes the maximum of every score once (two to a row, each of which has to know the whole row's
+// maximum, took it twice) and needs no exchange between the two at a tile's P (head size 128) and at an item's end.
+// Measured (one sequence, 32 / 8 heads; in brackets two threads to a row): head size 64, 333 tokens 15.2 us (17.4),
+// 2,048 44.5 (48.5), 4,096 135.5 (141.5), 8,192 482 (484), 16,384 1,778 (1,760); head size 128, 333 tokens 21.8 (26.4),
+// 2,048 70.6 (79.6), 8,192 837 (917), 16,384 3,149 (3,453).
+// Warp roles: warps 0-3 rows of slot 0, warps 4-7 rows of slot 1 (warp w owns TMEM lanes
+// 32 (w % 4) ..), warp 8 brings both Q tiles once per item and the K tiles, warp 9 the V tiles,
 // from the paged cache with 16-byte cp.async copies (zero-filled outside the live keys), lane 0
-// of warp 18 issues the MMAs of slot 0 and lane 0 of warp 19 those of slot 1 (a slot's products
+// of warp 10 issues the MMAs of slot 0 and lane 0 of warp 11 those of slot 1 (a slot's products
 // never wait for the other slot's rows).  Everything is handed over through mbarriers; every wait is
 // bounded (kSpinLimit polls), after which the CTA raises an abort flag, all roles leave their
 // loops, the copies in flight are waited for, TMEM is freed and bit 2 of *status is set.
@@ -41,7 +47,7 @@
 namespace rl {
 
 constexpr int kTcRows = 128, kTcKeys = 128;
-constexpr int kTcRowWarps = 16;                        // two threads to a row: 8 warps per slot
+constexpr int kTcRowWarps = 8;                         // a thread to a row: 4 warps per slot
 constexpr int kTcThreads = (kTcRowWarps + 4) * 32;      // the row warps, two loaders, two MMA warps
 constexpr int kTcHalves = kD / 64;                      // a head's columns in halves of 64 (128 bytes)
 constexpr int kTcHalfBytes = 128 * 128;                 // 128 rows x 64 bfloat16, 128-byte swizzled
@@ -60,8 +66,6 @@ struct PrefillTcShared {
   uint64_t qk_done[2], pv_done[2];                // per slot, MMA commits: S of the tile is ready / its O product is done
   uint64_t p_ready[2];                            // per slot: its four row warps have written P
   uint64_t s_free[2];                             // per slot: its four row warps have read S (used if P has its own columns)
-  uint64_t pair[2][4];                            // per slot and quarter of rows: the two warps that share the rows meet (2 arrivals)
-  float l_half[2][2][kTcRows];                    // [slot][half][row]: a thread's part of the row's denominator
   uint64_t o_free[2];                             // per slot: its four row warps have read the item's O
   uint32_t tmem_base;
   volatile int abort;
@@ -119,20 +123,37 @@ __device__ __forceinline__ void umma_bf16_ts(uint32_t tmem_d, uint32_t tmem_a, u
       : "memory");
 }
 
-// 16 consecutive 32-bit columns of this thread's TMEM lane, load (no wait) and store.
-__device__ __forceinline__ void tmem_ld16_issue(uint32_t taddr, uint32_t* r) {
+// 32 consecutive 32-bit columns of this thread's TMEM lane: asked for (r may not be touched yet), and there.  The
+// wait names the registers, so that nothing that reads them can be moved before it.
+__device__ __forceinline__ void tmem_ld32_issue(uint32_t taddr, uint32_t* r) {
   asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+      "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
+      "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
       : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
-        "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+        "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]), "=r"(r[16]),
+        "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]),
+        "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
       : "r"(taddr));
 }
-// 64 consecutive 32-bit columns of this thread's TMEM lane in one instruction (no wait).
-__device__ __forceinline__ void tmem_ld64_issue(uint32_t taddr, uint32_t* r) {
+__device__ __forceinline__ void tmem_wait_ld32(uint32_t* r) {
+  asm volatile("tcgen05.wait::ld.sync.aligned;"
+               : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(r[4]), "+r"(r[5]), "+r"(r[6]), "+r"(r[7]),
+                 "+r"(r[8]), "+r"(r[9]), "+r"(r[10]), "+r"(r[11]), "+r"(r[12]), "+r"(r[13]), "+r"(r[14]),
+                 "+r"(r[15]), "+r"(r[16]), "+r"(r[17]), "+r"(r[18]), "+r"(r[19]), "+r"(r[20]), "+r"(r[21]),
+                 "+r"(r[22]), "+r"(r[23]), "+r"(r[24]), "+r"(r[25]), "+r"(r[26]), "+r"(r[27]), "+r"(r[28]),
+                 "+r"(r[29]), "+r"(r[30]), "+r"(r[31])
+               :
+               : "memory");
+}
+// 16 columns read (the load and the wait), and stored.
+__device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t* r) {
   asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x64.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31, %32, %33, %34, %35, %36, %37, %38, %39, %40, %41, %42, %43, %44, %45, %46, %47, %48, %49, %50, %51, %52, %53, %54, %55, %56, %57, %58, %59, %60, %61, %62, %63}, [%64];"
-      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]), "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31]), "=r"(r[32]), "=r"(r[33]), "=r"(r[34]), "=r"(r[35]), "=r"(r[36]), "=r"(r[37]), "=r"(r[38]), "=r"(r[39]), "=r"(r[40]), "=r"(r[41]), "=r"(r[42]), "=r"(r[43]), "=r"(r[44]), "=r"(r[45]), "=r"(r[46]), "=r"(r[47]), "=r"(r[48]), "=r"(r[49]), "=r"(r[50]), "=r"(r[51]), "=r"(r[52]), "=r"(r[53]), "=r"(r[54]), "=r"(r[55]), "=r"(r[56]), "=r"(r[57]), "=r"(r[58]), "=r"(r[59]), "=r"(r[60]), "=r"(r[61]), "=r"(r[62]), "=r"(r[63])
-      : "r"(taddr));
+      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];\n"
+      "tcgen05.wait::ld.sync.aligned;"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
+        "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+      : "r"(taddr)
+      : "memory");
 }
 __device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t* r) {
   asm volatile(
@@ -141,7 +162,6 @@ __device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t* r) {
         "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
       : "memory");
 }
-__device__ __forceinline__ void tmem_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 __device__ __forceinline__ void tmem_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 
 // Two floats in one 64-bit register and the packed arithmetic on them (one instruction for two lanes).
@@ -169,16 +189,16 @@ __device__ __forceinline__ float max3(float a, float b, float c) {
   return d;
 }
 
-// Sets the scores of 64 keys that a row may not see to -inf: key j of them is live if jmin <= j <= jmax.
+// Sets the scores of 32 keys that a row may not see to -inf: key j of them is live if jmin <= j <= jmax.
 // Without a window (the same for all threads) there is no lower limit to test.
-__device__ __forceinline__ void tc_mask64(uint32_t* sr, int jmax, int jmin, bool window) {
+__device__ __forceinline__ void tc_mask32(uint32_t* sr, int jmax, int jmin, bool window) {
   if (!window) {
 #pragma unroll
-    for (int j = 0; j < 64; ++j)
+    for (int j = 0; j < 32; ++j)
       if (j > jmax) sr[j] = 0xff800000u;
   } else {
 #pragma unroll
-    for (int j = 0; j < 64; ++j)
+    for (int j = 0; j < 32; ++j)
       if (j > jmax || j < jmin) sr[j] = 0xff800000u;
   }
 }
@@ -250,10 +270,9 @@ prefill_attn_tc_kernel(const PrefillArgs<bf16> a, int tiles, int* status) {
       mbar_init(&sh->q_free[s], 1);
       mbar_init(&sh->qk_done[s], 1);
       mbar_init(&sh->pv_done[s], 1);
-      mbar_init(&sh->p_ready[s], 8);      // one arrival per row warp of the slot (its lanes meet first)
-      mbar_init(&sh->s_free[s], 8);
-      mbar_init(&sh->o_free[s], 8);
-      for (int qq = 0; qq < 4; ++qq) mbar_init(&sh->pair[s][qq], 2);
+      mbar_init(&sh->p_ready[s], 4);      // one arrival per row warp of the slot (its lanes meet first)
+      mbar_init(&sh->s_free[s], 4);
+      mbar_init(&sh->o_free[s], 4);
     }
     for (int b = 0; b < kTcStages; ++b) {
       mbar_init(&sh->k_full[b], 1);
@@ -278,7 +297,7 @@ prefill_attn_tc_kernel(const PrefillArgs<bf16> a, int tiles, int* status) {
   pdl_wait();        // q and the newest keys come from the kernels before this one
 
   if (warp == kTcRowWarps || warp == kTcRowWarps + 1) {
-    // ------------------------------------------------------------------ loaders: warp 8 K (and both Q), warp 9 V
+    // ------------------------------------------------------------------ loaders: one warp K (and both Q), one V
     const bool is_v = warp == kTcRowWarps + 1;
     const int ps_shift = __ffs(a.page_size) - 1, ps_mask = a.page_size - 1;
     const size_t head_stride = static_cast<size_t>(a.page_size) * kD;
@@ -384,7 +403,7 @@ prefill_attn_tc_kernel(const PrefillArgs<bf16> a, int tiles, int* status) {
     }
     hand_over(true);
   } else if (warp >= kTcRowWarps + 2) {
-    // ------------------------------------------------------------------ MMA issue: lane 0 of warp 10 for slot 0, of warp 11 for slot 1
+    // ------------------------------------------------------------------ MMA issue: lane 0 of one warp per slot
     // Each slot has an issuing thread of its own, so that neither slot's products ever wait for the
     // other slot's rows.  With columns of its own for P a slot's products go  S(0), S(1), O += P(0) V,
     // S(2), O += P(1) V, ...: the S product runs one key tile ahead of the rows; with P over S:
@@ -474,22 +493,20 @@ prefill_attn_tc_kernel(const PrefillArgs<bf16> a, int tiles, int* status) {
       }
     }
   } else {
-    // ------------------------------------------------------------------ the row threads, two to a row
-    // Warp w < 16: slot w / 8, half h = (w / 4) % 2, rows 32 (w % 4) .. + 32 of the slot's tile (the TMEM
-    // lanes a warp may touch).  A thread has the keys 64 h .. + 64 of every S tile, writes their P, and has
-    // the columns h D / 2 .. + D / 2 of O.  Both threads of a row take the maximum over the whole row (the
-    // other half is read from tensor memory for that alone, which is cheaper than an exchange), so both
-    // come to the same reference and the same decisions; each keeps the denominator of its own keys, and
-    // the two are added at the item's end (one exchange through shared memory).
-    const int s = warp >> 3, h = (warp >> 2) & 1, q = warp & 3;
+    // ------------------------------------------------------------------ the row threads, one to a row
+    // Warp w < 8: slot w / 4, rows 32 (w % 4) .. + 32 of the slot's tile (the TMEM lanes a warp may touch).  A thread
+    // reads its row of S in four pieces of 32 keys: 2 and 3 for the maximum alone, then 0 and 1, which stay in
+    // registers; then 2 and 3 come once more, behind the exponentials of 0 and 1.  (All 128 scores at once do not fit
+    // beside the rest: 168 registers a thread.)  S is free for the next product when piece 3 has landed again,
+    // half-way through the exponentials.
+    const int s = warp >> 2, q = warp & 3;
     const int r = q * 32 + lane;                         // row of the tile = TMEM lane
     const uint32_t lane_addr = static_cast<uint32_t>(q * 32) << 16;
     const uint32_t s_addr = tmem + lane_addr + s * kTcKeys;           // S
-    const uint32_t p_addr = (kTcOwnP ? tmem + lane_addr + kTcColP + s * 64 : s_addr) + h * 32;   // this thread's 32 columns of P
-    const uint32_t o_addr = tmem + lane_addr + kTcColO + s * kD + h * (kD / 2);
+    const uint32_t p_addr = kTcOwnP ? tmem + lane_addr + kTcColP + s * 64 : s_addr;      // 64 columns of P
+    const uint32_t o_addr = tmem + lane_addr + kTcColO + s * kD;
     const float sc = a.scale * kLog2e;
     bool ok = true;
-    int xphase = 0;                                       // exchanges done so far (parity of the pair's mbarrier)
     TcWalk wk;
     for (bool more = wk.first(a, n_items, pairs, tiles); more && ok; more = wk.next(a, n_items, pairs, tiles)) {
       const TcItem& w = wk.w;
@@ -499,7 +516,7 @@ prefill_attn_tc_kernel(const PrefillArgs<bf16> a, int tiles, int* status) {
       const int pos_r = pos0 + r;
       const int win_r = (a.window > 0 && pos_r + 1 > a.window) ? pos_r + 1 - a.window : 0;
       const int lim_r = r < rows ? pos_r : -1;             // the row's live keys are win_r .. lim_r (none for a row past the tile's rows)
-      float m_ref = -INFINITY, l = 0.f;                   // the maximum that P is scaled by (log2 units), this thread's part of the denominator
+      float m_ref = -INFINITY, l = 0.f;                   // the maximum that P is scaled by (log2 units), the denominator
       for (int i = 0; i < w.nt && ok; ++i) {
         const int n = g_base + i;
         const int t0 = w.k_begin + i * kTcKeys;
@@ -511,33 +528,37 @@ prefill_attn_tc_kernel(const PrefillArgs<bf16> a, int tiles, int* status) {
         // tile's rows need the masks (the same for the whole CTA)
         const bool masked = (t0 + kTcKeys - 1 > pos0) || (a.window > 0 && t0 < pos0 + kTcRows - a.window) || (rows < kTcRows);
         float mx0 = -INFINITY, mx1 = -INFINITY;
-        uint32_t sr[64];
-        {   // the other thread's keys, for the maximum; then this thread's own
-          tmem_ld64_issue(s_addr + (h ^ 1) * 64, sr);
-          tmem_wait_ld();
-          if (masked) tc_mask64(sr, lim_r - (t0 + (h ^ 1) * 64), win_r - (t0 + (h ^ 1) * 64), a.window > 0);
+        auto mask = [&](uint32_t* v, int piece) {
+          if (masked) tc_mask32(v, lim_r - (t0 + piece * 32), win_r - (t0 + piece * 32), a.window > 0);
+        };
+        auto maximum = [&](const uint32_t* v) {
 #pragma unroll
-          for (int j = 0; j < 64; j += 4) {
-            mx0 = max3(mx0, __uint_as_float(sr[j]), __uint_as_float(sr[j + 1]));
-            mx1 = max3(mx1, __uint_as_float(sr[j + 2]), __uint_as_float(sr[j + 3]));
+          for (int j = 0; j < 32; j += 4) {
+            mx0 = max3(mx0, __uint_as_float(v[j]), __uint_as_float(v[j + 1]));
+            mx1 = max3(mx1, __uint_as_float(v[j + 2]), __uint_as_float(v[j + 3]));
           }
-        }
-        tmem_ld64_issue(s_addr + h * 64, sr);
-        tmem_wait_ld();
-        if (kTcOwnP) {                                     // S is in registers: the next S product may overwrite it
-          tc_fence_before();
-          __syncwarp();
-          if (lane == 0) mbar_arrive(&sh->s_free[s]);
-        }
-        if (masked) tc_mask64(sr, lim_r - (t0 + h * 64), win_r - (t0 + h * 64), a.window > 0);
-#pragma unroll
-        for (int j = 0; j < 64; j += 4) {
-          mx0 = max3(mx0, __uint_as_float(sr[j]), __uint_as_float(sr[j + 1]));
-          mx1 = max3(mx1, __uint_as_float(sr[j + 2]), __uint_as_float(sr[j + 3]));
-        }
+        };
+        uint32_t va[32], vb[32], vc[32];
+        tmem_ld32_issue(s_addr + 64, vc);
+        tmem_wait_ld32(vc);
+        tmem_ld32_issue(s_addr + 96, vb);
+        mask(vc, 2);
+        maximum(vc);
+        tmem_wait_ld32(vb);
+        tmem_ld32_issue(s_addr, va);
+        mask(vb, 3);
+        maximum(vb);
+        tmem_wait_ld32(va);
+        tmem_ld32_issue(s_addr + 32, vb);
+        mask(va, 0);
+        maximum(va);
+        tmem_wait_ld32(vb);
+        tmem_ld32_issue(s_addr + 64, vc);                 // once more, for P: waited for when piece 0 has become P
+        mask(vb, 1);
+        maximum(vb);
         const float m_new = fmaxf(m_ref, fmaxf(mx0, mx1) * sc);   // in units of log2 of the scaled scores
-        // The reference moves for the whole warp or not at all (the other warp of these rows sees the same
-        // maxima and decides the same); the denominator follows at once, the row of O below, when O is at rest.
+        // The reference moves for the whole warp or not at all; the denominator follows at once, the row of O below,
+        // when O is at rest.
         float alpha = 1.f;
         bool moved = false;
         if (i == 0) {
@@ -551,89 +572,82 @@ prefill_attn_tc_kernel(const PrefillArgs<bf16> a, int tiles, int* status) {
         const float m_use = m_ref == -INFINITY ? 0.f : m_ref;  // a row without a live key so far
         const uint64_t sc2 = f32x2(sc, sc), nm2 = f32x2(-m_use, -m_use);
         uint64_t sum_a = f32x2(0.f, 0.f), sum_b = sum_a;
+        // 32 scores become 16 columns of P (two keys to a column)
+        auto exponentials = [&](uint32_t* v) {
 #pragma unroll
-        for (int j = 0; j < 64; j += 4) {
-          float x0, x1, x2, x3;
-          f32x2_split(fma_f32x2(f32x2(__uint_as_float(sr[j]), __uint_as_float(sr[j + 1])), sc2, nm2), x0, x1);
-          f32x2_split(fma_f32x2(f32x2(__uint_as_float(sr[j + 2]), __uint_as_float(sr[j + 3])), sc2, nm2), x2, x3);
-          const float p0 = ex2_approx(x0), p1 = ex2_approx(x1), p2 = ex2_approx(x2), p3 = ex2_approx(x3);
-          sum_a = add_f32x2(sum_a, f32x2(p0, p1));
-          sum_b = add_f32x2(sum_b, f32x2(p2, p3));
-          const __nv_bfloat162 lo = __floats2bfloat162_rn(p0, p1), hi = __floats2bfloat162_rn(p2, p3);
-          sr[j >> 1] = *reinterpret_cast<const uint32_t*>(&lo);       // (columns j / 2: behind the ones still to be read)
-          sr[(j >> 1) + 1] = *reinterpret_cast<const uint32_t*>(&hi);
+          for (int j = 0; j < 32; j += 4) {
+            float x0, x1, x2, x3;
+            f32x2_split(fma_f32x2(f32x2(__uint_as_float(v[j]), __uint_as_float(v[j + 1])), sc2, nm2), x0, x1);
+            f32x2_split(fma_f32x2(f32x2(__uint_as_float(v[j + 2]), __uint_as_float(v[j + 3])), sc2, nm2), x2, x3);
+            const float p0 = ex2_approx(x0), p1 = ex2_approx(x1), p2 = ex2_approx(x2), p3 = ex2_approx(x3);
+            sum_a = add_f32x2(sum_a, f32x2(p0, p1));
+            sum_b = add_f32x2(sum_b, f32x2(p2, p3));
+            const __nv_bfloat162 lo = __floats2bfloat162_rn(p0, p1), hi = __floats2bfloat162_rn(p2, p3);
+            v[j >> 1] = *reinterpret_cast<const uint32_t*>(&lo);       // (columns j / 2: behind the ones still to be read)
+            v[(j >> 1) + 1] = *reinterpret_cast<const uint32_t*>(&hi);
+          }
+        };
+        exponentials(va);
+        if (kTcOwnP && n > 0) {
+          // P of the tile before must have been read, and O must be at rest, before this tile's P and a
+          // rescaled O are written (with P over S, the product that made S waited for that)
+          ok = mbar_wait(&sh->pv_done[s], (n - 1) & 1, &sh->abort);
+          ok = __all_sync(0xffffffffu, ok);
+          tc_fence_after();
         }
+        tmem_wait_ld32(vc);
+        if (!ok) break;
+        if (moved) {
+#pragma unroll 1
+          for (int c0 = 0; c0 < kD; c0 += 16) {
+            uint32_t o[16];
+            tmem_ld16(o_addr + c0, o);
+#pragma unroll
+            for (int d = 0; d < 16; ++d) o[d] = __float_as_uint(__uint_as_float(o[d]) * alpha);
+            tmem_st16(o_addr + c0, o);
+          }
+        }
+        // (P over S: the columns of P's pieces are those of S's pieces 0 and 1, which have been read)
+        tmem_st16(p_addr, va);
+        tmem_ld32_issue(s_addr + 96, va);
+        exponentials(vb);
+        tmem_wait_ld32(va);
+        if (kTcOwnP) {                                     // S is in registers: the next S product may overwrite it
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&sh->s_free[s]);
+        }
+        tmem_st16(p_addr + 16, vb);
+        mask(vc, 2);
+        exponentials(vc);
+        tmem_st16(p_addr + 32, vc);
+        mask(va, 3);
+        exponentials(va);
+        tmem_st16(p_addr + 48, va);
         {
           float s0, s1, s2, s3;
           f32x2_split(sum_a, s0, s1);
           f32x2_split(sum_b, s2, s3);
           l += (s0 + s1) + (s2 + s3);
         }
-        if (kTcOwnP && n > 0) {
-          // P of the tile before must have been read, and O must be at rest, before this tile's P and a
-          // rescaled O are written (long done by now: that product was issued a whole tile ago)
-          ok = mbar_wait(&sh->pv_done[s], (n - 1) & 1, &sh->abort);
-          ok = __all_sync(0xffffffffu, ok);
-          if (!ok) break;
-          tc_fence_after();
-        }
-        if (!kTcOwnP) {
-          // P goes over columns of S that the other thread of the row reads too (its own keys, or this
-          // thread's for the maximum): both must have read S before either writes P
-          tc_fence_before();
-          __syncwarp();
-          if (lane == 0) mbar_arrive(&sh->pair[s][q]);
-          ok = mbar_wait(&sh->pair[s][q], xphase & 1, &sh->abort);
-          ++xphase;
-          ok = __all_sync(0xffffffffu, ok);
-          if (!ok) break;
-          tc_fence_after();
-        }
-        if (moved) {
-          // (with P over S, O is at rest too: the product that made S waited for the O product of the tile before)
-#pragma unroll
-          for (int c0 = 0; c0 < kD / 2; c0 += 32) {
-            uint32_t o[32];
-            tmem_ld16_issue(o_addr + c0, o);
-            tmem_ld16_issue(o_addr + c0 + 16, o + 16);
-            tmem_wait_ld();
-#pragma unroll
-            for (int d = 0; d < 32; ++d) o[d] = __float_as_uint(__uint_as_float(o[d]) * alpha);
-            tmem_st16(o_addr + c0, o);
-            tmem_st16(o_addr + c0 + 16, o + 16);
-          }
-        }
-        // P: two keys per 32-bit column; this thread's 64 keys are 32 columns
-        tmem_st16(p_addr, sr);
-        tmem_st16(p_addr + 16, sr + 16);
         tmem_wait_st();
         tc_fence_before();
         __syncwarp();
         if (lane == 0) mbar_arrive(&sh->p_ready[s]);
       }
       if (!ok) break;
-      // ---- the row's denominator: this thread's part and the other's
-      sh->l_half[s][h][r] = l;
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&sh->pair[s][q]);        // (release: the values are visible to who sees the phase)
-      ok = mbar_wait(&sh->pair[s][q], xphase & 1, &sh->abort);
-      ++xphase;
-      ok = __all_sync(0xffffffffu, ok);
-      if (!ok) break;
-      const float l_all = l + sh->l_half[s][h ^ 1][r];
       // ---- the item's rows: O / denominator, once its last product is done
       ok = mbar_wait(&sh->pv_done[s], (g_base + w.nt - 1) & 1, &sh->abort);
       ok = __all_sync(0xffffffffu, ok);
       if (!ok) break;
       tc_fence_after();
-      const float inv = l_all > 0.f ? 1.f / l_all : 0.f;
-      bf16* dst = a.out + static_cast<size_t>(w.tok0 + (r < rows ? r : 0)) * a.out_stride + (w.head0 + s) * kD + h * (kD / 2);
+      const float inv = l > 0.f ? 1.f / l : 0.f;
+      bf16* dst = a.out + static_cast<size_t>(w.tok0 + (r < rows ? r : 0)) * a.out_stride + (w.head0 + s) * kD;
 #pragma unroll
-      for (int c0 = 0; c0 < kD / 2; c0 += 32) {
+      for (int c0 = 0; c0 < kD; c0 += 32) {
         uint32_t o[32];
-        tmem_ld16_issue(o_addr + c0, o);
-        tmem_ld16_issue(o_addr + c0 + 16, o + 16);
-        tmem_wait_ld();
+        tmem_ld32_issue(o_addr + c0, o);
+        tmem_wait_ld32(o);
         if (r < rows) {
 #pragma unroll
           for (int d = 0; d < 32; d += 8) {
