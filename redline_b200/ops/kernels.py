@@ -514,9 +514,13 @@ def attn_decode_rows_pays(nitems: int, num_kv_heads: int, head_dim: int, max_ctx
     a launch of ``nitems`` rows of at most ``max_ctx`` and together ``sum_ctx`` keys.  Its time goes with the
     longest row (a row has its cluster's SMs only) times the rows a cluster takes in turn, the streaming
     kernel's with all keys plus the count and merge of its pieces.  The constants are fitted to times on a
-    B200 (head size 64, 8 kv heads, batches 1 to 128 at 512 to 8,192 keys): 4.4 us plus, per row a group of
-    warps takes, 1.7 us per 32-key sub-block of a warp's run (and 0.7 + 0.25 x turns when it takes more than
-    one), but no less than the keys' bytes at 6.2 TB/s; against 8 us plus the keys' bytes at 5.3 TB/s."""
+    B200 (8 kv heads, head sizes 64 and 128, batches of 1 to 64 with 512 to 4,000 keys: equal lengths, lengths spread
+    over L / 8 to L, and one long row among short ones): 3.5 us plus 0.7 us (head size 64) per 32-key sub-block of a
+    warp's run, but no less than the keys' bytes at 6.2 TB/s, plus 0.8 us (less below 1,024 keys) for every mean
+    length that the longest row has beyond one; against 8 us plus the keys' bytes at 3 TB/s.  Over 108 such launches the
+    choice is off by 27 us in all at head size 64 and by 15 us at 128 (constants fitted to equal lengths at head size 64 alone, 4.4 + 1.7 and 8 + bytes
+    at 5.3 TB/s: 68 and 575 us).  21 sequences of 115 to 925 keys: 9.5 us against 13.6; eight of 4,000 at head size 128:
+    25 against 36."""
     csize, resident = attn_decode_rows_cluster(nitems, num_kv_heads, head_dim, device)
     if csize <= 0 or resident <= 0 or max_ctx <= 0:
         return False
@@ -533,9 +537,10 @@ def attn_decode_rows_pays(nitems: int, num_kv_heads: int, head_dim: int, max_ctx
     sub_blocks = (max_ctx + 31) // 32
     per_row = csize * (warps // groups)
     nbytes = sum_ctx * num_kv_heads * head_dim * 4
-    per_turn = 1.7 * (head_dim / 64.0) * ((sub_blocks + per_row - 1) // per_row) + (0.7 + 0.25 * turns if turns > 1 else 0.0)
-    t_rows = 4.4 + max(turns * per_turn, nbytes / 6.2e6)
-    t_stream = 8.0 + nbytes / 5.3e6
+    run = turns * ((sub_blocks + per_row - 1) // per_row) * (head_dim / 64.0)
+    t_rows = 3.5 + max(0.7 * run, nbytes / 6.2e6)
+    t_rows += 0.8 * (max_ctx * nitems / max(sum_ctx, 1) - 1.0) * min(1.0, max_ctx / 1024.0)
+    t_stream = 8.0 + nbytes / 3.0e6
     return t_rows < t_stream
 
 

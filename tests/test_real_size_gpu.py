@@ -237,3 +237,33 @@ def test_generation_with_graphs_and_tokens_fed_on_the_device(dtype, models):
         check(got, want, dtype, f"request {o['id']}")
         assert [int(g.argmax()) for g in got] == o["output_ids"]
     eng.runner.check_status()
+
+
+@pytest.mark.parametrize("lens", [[925 - 38 * i for i in range(21)], [2000, 1200, 700, 300] * 3])
+def test_spread_lengths_take_a_cluster_per_row(lens):
+    """Lengths spread over a factor of five to eight: the rows kernel is named, and it and the streaming kernel agree
+    (bfloat16 outputs of two orders of summation: a few ulps of the largest)."""
+    from redline_b200.ops import kernels
+    dev = torch.device("cuda")
+    Hq, Hkv, D, ps, n = 32, 8, 64, 16, len(lens)
+    assert kernels.attn_decode_rows_pays(n, Hkv, D, max(lens), sum(lens), 0, dev)
+    g = torch.Generator().manual_seed(5)
+    pages = [(x + ps - 1) // ps for x in lens]
+    kc, vc = (torch.randn(sum(pages) + 1, Hkv, ps, D, generator=g).to(torch.bfloat16).to(dev) for _ in range(2))
+    table, at = torch.zeros(n, max(pages), dtype=torch.int32), 1
+    for i, p in enumerate(pages):
+        table[i, :p] = torch.arange(at, at + p)
+        at += p
+    table = table.to(dev)
+    q = torch.randn(n, Hq * D, generator=g).to(torch.bfloat16).to(dev)
+    items = torch.tensor([[i, i, x, 0] for i, x in enumerate(lens)], dtype=torch.int32, device=dev)
+    parts = (max(lens) + kernels.DECODE_PARTITION - 1) // kernels.DECODE_PARTITION
+    part_o, part_ml = torch.empty(n * Hq * parts * D, device=dev), torch.empty(n * Hq * parts * 2, device=dev)
+    counters = torch.zeros(n * Hkv, dtype=torch.int32, device=dev)
+    outs = []
+    for impl in (4, 3):
+        out = torch.zeros(n, Hq * D, dtype=torch.bfloat16, device=dev)
+        kernels.attn_decode(q, q.stride(0), kc, vc, table, items, part_o, part_ml, parts, counters, out, n, Hq, Hkv, D, ps,
+                            0, D ** -0.5, impl)
+        outs.append(out.float())
+    assert (outs[0] - outs[1]).abs().max() <= 2.0 ** -7 * outs[1].abs().max()
