@@ -134,8 +134,8 @@ struct Piece<T, 1> {
 //
 // A launch is a few keys to each SM (eight sequences of 540 keys, 4 kv heads: 160 CTAs with 64 KB each), so what
 // bounds it is the chain of round trips to memory, not bytes.  A thread therefore asks for all its pieces of the partition's
-// keys AND values before it multiplies any (16 pieces of each where rows have 128 entries or less in 16 bits; longer rows
-// in batches), and reads the work item and its pages while the kernel before still runs.  Decode steps of eight such
+// keys AND values before it multiplies any (16 pieces of each where rows have 128 entries or less in 16 bits; rows of up
+// to 256 in batches of four; of longer rows a piece when it is multiplied: the sums alone take the registers there), and reads the work item and its pages while the kernel before still runs.  Decode steps of eight such
 // sequences, with the merge below: 0.52 -> 0.48 ms (two layers of 64 / 128 entries and two maps), 0.36 -> 0.31 ms (three of
 // 128 / 128 and 96 entries).
 template <typename T>
@@ -150,11 +150,13 @@ maps_decode_kernel(const MapsDecodeArgs<T> a) {
   constexpr int CHV = kDV / EVV;
   constexpr int CPLV = (CHV + kLPK - 1) / kLPK;
   constexpr int IT = kPart / kKeysPerIter;               // keys of a thread
-  constexpr int KB = CPL <= 2 ? IT : (CPL <= 4 ? 4 : (CPL <= 8 ? 2 : 1));                // ... asked for at once
-  constexpr int VB = CPLV <= 2 ? IT : (CPLV <= 4 ? 4 : (CPLV <= 8 ? 2 : 1));                 // ... values
+  constexpr int KB = CPL <= 2 ? IT : (CPL <= 4 ? 4 : 1);                                    // ... asked for at once
+  constexpr int VB = CPLV <= 2 ? IT : (CPLV <= 4 ? 4 : 1);                                  // ... values
   constexpr bool kValuesAhead = VB == IT;                // the partition's values are asked for with its keys
   static_assert(IT % KB == 0 && IT % VB == 0, "whole batches");
-  __shared__ __align__(16) float qs[kM][kRows][kD];
+  // (the rows of both maps at once where static shared memory has room for them)
+  constexpr int kQM = kM * kRows * kD + kRows * kPart + kThreads / 32 * kRows * kDV + 2 * kRows <= 12288 ? kM : 1;
+  __shared__ __align__(16) float qs[kQM][kRows][kD];
   __shared__ float sc[kRows][kPart];
   __shared__ float red[kThreads / 32][kRows][kDV];
   __shared__ float stat_m[kRows], stat_l[kRows];
@@ -191,12 +193,20 @@ maps_decode_kernel(const MapsDecodeArgs<T> a) {
   }
   pdl_wait();         // q and the newest keys and values come from the kernels before this one
 
-  Piece<T, E> kr[KB][CPL];
+  auto key_row = [&](int m, int it) {
+    const int j = base + it * kKeysPerIter + slot;
+    return a.kcache + ((static_cast<size_t>(pages[it]) * (a.kv_heads * kM) + kvh * kM + m) * a.page_size + j % a.page_size) * kD;
+  };
+  auto value_row = [&](int it) {
+    const int j = base + it * kKeysPerIter + slot;
+    return a.vcache + ((static_cast<size_t>(pages[it]) * a.kv_heads + kvh) * a.page_size + j % a.page_size) * kVS;
+  };
+  Piece<T, E> kr[KB][KB > 1 ? CPL : 1];
   auto ask_keys = [&](int m, int it0) {
 #pragma unroll
     for (int b = 0; b < KB; ++b) {
-      const int it = it0 + b, j = base + it * kKeysPerIter + slot;
-      const T* kp = a.kcache + ((static_cast<size_t>(pages[it]) * (a.kv_heads * kM) + kvh * kM + m) * a.page_size + j % a.page_size) * kD;
+      const int it = it0 + b;
+      const T* kp = key_row(m, it);
 #pragma unroll
       for (int c = 0; c < CPL; ++c) {
         const int ch = lane8 + c * kLPK;
@@ -205,12 +215,12 @@ maps_decode_kernel(const MapsDecodeArgs<T> a) {
       }
     }
   };
-  Piece<T, EVV> vr[VB][CPLV];
+  Piece<T, EVV> vr[VB][VB > 1 ? CPLV : 1];
   auto ask_values = [&](int it0) {
 #pragma unroll
     for (int b = 0; b < VB; ++b) {
-      const int it = it0 + b, j = base + it * kKeysPerIter + slot;
-      const T* vp = a.vcache + ((static_cast<size_t>(pages[it]) * a.kv_heads + kvh) * a.page_size + j % a.page_size) * kVS;
+      const int it = it0 + b;
+      const T* vp = value_row(it);
 #pragma unroll
       for (int c = 0; c < CPLV; ++c) {
         const int ch = lane8 + c * kLPK;
@@ -219,20 +229,29 @@ maps_decode_kernel(const MapsDecodeArgs<T> a) {
       }
     }
   };
-  ask_keys(0, 0);
-  for (int i = threadIdx.x; i < kM * kRows * kD; i += kThreads) {
-    const int m = i / (kRows * kD), g = (i - m * (kRows * kD)) / kD, d = i % kD;
-    qs[m][g][d] = g < ng ? to_float(a.q[static_cast<size_t>(tok) * a.q_stride + ((kvh * G + g0 + g) * kM + m) * kD + d]) * a.scale
-                         : 0.f;
-  }
-  if (kValuesAhead) ask_values(0);
+  if constexpr (KB > 1) ask_keys(0, 0);
+  auto load_q = [&](int m0) {
+    for (int i = threadIdx.x; i < kQM * kRows * kD; i += kThreads) {
+      const int m = i / (kRows * kD), g = (i - m * (kRows * kD)) / kD, d = i % kD;
+      qs[m][g][d] = g < ng ? to_float(a.q[static_cast<size_t>(tok) * a.q_stride + ((kvh * G + g0 + g) * kM + m0 + m) * kD + d]) * a.scale
+                           : 0.f;
+    }
+  };
+  load_q(0);
+  if constexpr (kValuesAhead) ask_values(0);
   __syncthreads();
 
   for (int m = 0; m < kM; ++m) {
+    if (kQM < kM && m > 0) {         // (the rows of the map before are out of use since its scores)
+      load_q(m);
+      __syncthreads();
+    }
     // ---- scores (every lane of a warp makes the same number of trips: the shuffles need all of them)
 #pragma unroll
     for (int it0 = 0; it0 < IT; it0 += KB) {
-      if (KB < IT && (m > 0 || it0 > 0)) ask_keys(m, it0);
+      if constexpr (KB > 1 && KB < IT) {
+        if (m > 0 || it0 > 0) ask_keys(m, it0);
+      }
 #pragma unroll
       for (int b = 0; b < KB; ++b) {
         const int it = it0 + b, j = base + it * kKeysPerIter + slot;
@@ -242,13 +261,14 @@ maps_decode_kernel(const MapsDecodeArgs<T> a) {
 #pragma unroll
         for (int c = 0; c < CPL; ++c) {
           const int ch = lane8 + c * kLPK;
-          if (CH % kLPK == 0 || ch < CH) {
+          if (KB > 1 ? CH % kLPK == 0 || ch < CH : (live >> it & 1) && ch < CH) {
             float kf[E];
-            kr[b][c].get(kf);
+            if (KB == 1) kr[0][0].load(key_row(m, it) + ch * E);
+            kr[b][KB > 1 ? c : 0].get(kf);
 #pragma unroll
             for (int g = 0; g < kRows; ++g) {
 #pragma unroll
-              for (int e = 0; e < E; ++e) dot[g] += kf[e] * qs[m][g][ch * E + e];
+              for (int e = 0; e < E; ++e) dot[g] += kf[e] * qs[kQM < kM ? 0 : m][g][ch * E + e];
             }
           }
         }
@@ -262,7 +282,9 @@ maps_decode_kernel(const MapsDecodeArgs<T> a) {
         }
       }
     }
-    if (KB == IT && m + 1 < kM) ask_keys(m + 1, 0);
+    if constexpr (KB == IT) {
+      if (m + 1 < kM) ask_keys(m + 1, 0);
+    }
     __syncthreads();
     // ---- cap, slopes and softmax statistics of this partition, one warp per row, a lane per key and 32 more
     for (int g = warp; g < ng; g += kThreads / 32) {
@@ -305,7 +327,7 @@ maps_decode_kernel(const MapsDecodeArgs<T> a) {
         for (int e = 0; e < EVV; ++e) acc[g][c][e] = 0.f;
 #pragma unroll
     for (int it0 = 0; it0 < IT; it0 += VB) {
-      if (!kValuesAhead) ask_values(it0);
+      if constexpr (VB > 1 && !kValuesAhead) ask_values(it0);
 #pragma unroll
       for (int b = 0; b < VB; ++b) {
         const int it = it0 + b;
@@ -315,8 +337,11 @@ maps_decode_kernel(const MapsDecodeArgs<T> a) {
         for (int g = 0; g < kRows; ++g) p[g] = g < ng ? sc[g][it * kKeysPerIter + slot] : 0.f;
 #pragma unroll
         for (int c = 0; c < CPLV; ++c) {
+          const int ch = lane8 + c * kLPK;
+          if (VB == 1 && ch >= CHV) continue;
           float vf[EVV];
-          vr[b][c].get(vf);
+          if (VB == 1) vr[0][0].load(value_row(it) + ch * EVV);
+          vr[b][VB > 1 ? c : 0].get(vf);
 #pragma unroll
           for (int g = 0; g < kRows; ++g)
 #pragma unroll

@@ -306,3 +306,11 @@ def test_attention_with_maps_over_shuffled_pages(dtype, H, G, M, D, DV, size, ke
     kernels.maps_attn_decode(qd, qd.stride(0), kc, vc, table, items, part_o, part_ml, parts, out, len(ends), H, G, D, DV,
                              M, ps, size, keep, scale, cap, lam, post, eps, True)
     assert rel(out[rows], want[rows]) < tol
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("H,G,M,D,DV", [(2, 1, 2, 75, 70), (4, 2, 1, 200, 144), (2, 1, 2, 568, 504)])
+def test_attention_with_maps_over_long_rows(dtype, H, G, M, D, DV):
+    """Rows of which a thread asks for four keys at a time, or for a piece when it is multiplied, and queries of two maps
+    that shared memory holds one after the other."""
+    test_attention_with_maps_over_shuffled_pages(dtype, H, G, M, D, DV, 24, 3, 12.0)
