@@ -908,3 +908,20 @@ def test_gemm_tc_refuses_what_it_cannot_do():
     assert not kernels.gemm_tc_ok(x, w)
     with pytest.raises(kernels.KernelError):
         kernels.gemm_tc(x, w, torch.zeros(4, 32, device=DEV, dtype=torch.bfloat16))
+
+
+@pytest.mark.parametrize("M", [65, 73, 81, 96, 105, 113, 121, 128])
+def test_simt_product_with_a_short_last_tile(M):
+    """Every number of eights of rows that the last 64-row tile of a float32 product can have: float64 within the rounding
+    of 1,030 ordered sums, and the bits that the same rows have in a product of 16 rows."""
+    from redline_b200.ops import kernels
+    N, K = 3100, 1028
+    g = torch.Generator().manual_seed(M)
+    x, w = torch.randn(M, K, generator=g).cuda(), torch.randn(N, K, generator=g).cuda()
+    y, few = torch.empty(M, N, device="cuda"), torch.empty(16, N, device="cuda")
+    kernels.gemm_tn_simt(x, w, y)
+    kernels.gemm_tn_simt(x[M - 16:], w, few)
+    want = x.double() @ w.double().T
+    bound = (x.abs().double() @ w.abs().double().T) * (K / 8 + 8) * 2.0 ** -24
+    assert ((y.double() - want).abs() <= bound).all()
+    assert torch.equal(y[M - 16:], few)
