@@ -1628,6 +1628,7 @@ def build_all(head_dims=(64, 128), maps_dims=((64, 128, 2), (128, 128, 1)), line
     jobs += [(f"matrix_memory_d{d}", "matrix_memory.cu", {"RL_MM_DIM": d}) for d in memory_dims]
     jobs += [(f"state_space_d{d}", "linear_attention.cu", {"RL_LIN_DIM": d, "RL_LIN_TOKEN": 1}) for d in state_dims]
     jobs += [(f"delta_rule_d{d}", "delta_rule.cu", {"RL_DELTA_DIM": d}) for d in delta_dims]
+    build.build_dir()          # (decided once, before the threads: each would probe the folder with the same file)
     with ThreadPoolExecutor(max(1, min(8, os.cpu_count() or 1))) as pool:
         built = list(pool.map(lambda job: build.compile_module(*job, verbose=verbose), jobs))
     build.remove_other_versions(built)
