@@ -225,6 +225,15 @@ sample_partial_kernel(const float* __restrict__ logits, int vocab, int ld, Chunk
   if (threadIdx.x == 0) stats[row * kSampleChunks + chunk] = ChunkStat{b.v, b.i, s, 0.f};
 }
 
+// A row's result (one thread).  A row of which no logit is above -inf (all -inf, or NaN) has no best token: it gets
+// token 0 and the log-probability NaN, and nothing is read at the index that stands for "none".
+__device__ __forceinline__ void write_draw(const float* l, int token, float lse, int row, int32_t* out_token,
+                                           float* out_logprob) {
+  const bool found = token != 0x7fffffff;
+  out_token[row] = found ? token : 0;
+  if (out_logprob) out_logprob[row] = found ? l[token] - lse : NAN;
+}
+
 // Greedy row with first-stage statistics, by one warp: combine the pieces (smaller index wins ties).
 __device__ __forceinline__ void greedy_from_stats(const float* l, const ChunkStat* stats, int row,
                                                   int32_t* out_token, float* out_logprob) {
@@ -246,10 +255,7 @@ __device__ __forceinline__ void greedy_from_stats(const float* l, const ChunkSta
     if (st.idx != 0x7fffffff) sum += st.sumexp * expf(st.mx - b.v);
   }
   sum = warp_sum(sum);
-  if (threadIdx.x == 0) {
-    out_token[row] = b.i;
-    if (out_logprob) out_logprob[row] = l[b.i] - (b.v + logf(sum));
-  }
+  if (threadIdx.x == 0) write_draw(l, b.i, b.v + logf(sum), row, out_token, out_logprob);
 }
 
 __global__ void __launch_bounds__(kSampleThreads)
@@ -315,10 +321,7 @@ sample_kernel(const float* __restrict__ logits, int vocab, int ld, const float* 
     g = block_best(g, sh.bscratch);
     if (g.i != 0x7fffffff) token = g.i;
   }
-  if (threadIdx.x == 0) {
-    out_token[row] = token;
-    if (out_logprob) out_logprob[row] = l[token] - lse;
-  }
+  if (threadIdx.x == 0) write_draw(l, token, lse, row, out_token, out_logprob);
 }
 
 // ---------------------------------------------------------------- sampled rows of a large vocabulary
@@ -544,10 +547,7 @@ sample_cluster_kernel(const float* __restrict__ logits, int vocab, int ld, const
     g = cluster_best(block_best(g, sh.bscratch), &sh.best);
     if (g.i != 0x7fffffff) token = g.i;
   }
-  if (rank == 0 && threadIdx.x == 0) {
-    out_token[row] = token;
-    if (out_logprob) out_logprob[row] = l[token] - lse;
-  }
+  if (rank == 0 && threadIdx.x == 0) write_draw(l, token, lse, row, out_token, out_logprob);
   cluster_meet();                                  // (no CTA ends while a peer may read its shared memory)
 }
 

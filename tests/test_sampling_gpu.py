@@ -122,6 +122,20 @@ def test_draw_over_a_cluster_equals_the_plain_restatement(V, ld, T, k, p):
     assert np.abs(lp - want.numpy()).max() < 1e-4
 
 
+@pytest.mark.parametrize("two_stage", [False, True])
+@pytest.mark.parametrize("V", [1, 331, 8191, 8192, 20001, 128256])
+def test_rows_without_a_best_logit(V, two_stage):
+    """Rows of NaN and of -inf only, greedy and sampled (in one block and over a cluster): token 0 and a NaN
+    log-probability; the rows beside them are drawn as ever."""
+    l = torch.randn(6, V, device=DEV)
+    l[0], l[1], l[3], l[4] = float("nan"), -float("inf"), float("nan"), -float("inf")
+    temp = np.array([0.0, 0.0, 0.0, 0.8, 0.8, 0.8], dtype=np.float32)
+    tok, lp = run(l, temp, 5 if V > 5 else 0, 0.9, 7, np.arange(6), two_stage)
+    assert tok[[0, 1, 3, 4]].tolist() == [0] * 4 and np.isnan(lp[[0, 1, 3, 4]]).all()
+    assert tok[2] == int(l[2].argmax()) and np.isfinite(lp[[2, 5]]).all()
+    assert tok[5] == P.gumbel_draw(l[5].cpu().numpy(), 0.8, 5 if V > 5 else 0, 0.9, 7, 5)
+
+
 @pytest.mark.parametrize("V", [1, 511, 4096, 50001])
 def test_gather_logprob_one_pass(V):
     """Rows shorter than a block's first loads, on its edge, and ragged; values far apart and -inf."""
