@@ -133,18 +133,18 @@ __device__ __forceinline__ void tc_drain(const TcArgs& a, uint32_t acc, int row,
             for (int i = 0; i < 32 && n0 + c + i < a.N; ++i) out[i] = v[i];
           }
         } else {
-          float* out = static_cast<float*>(a.y) + o;   // residual += bfloat16(product)
+          float* out = static_cast<float*>(a.y) + o;   // residual += product, both float32
           if (whole && (a.ldy % 4 == 0)) {
 #pragma unroll
             for (int i = 0; i < 32; i += 4) {
               float r4[4];
               load16(out + i, r4);
 #pragma unroll
-              for (int e = 0; e < 4; ++e) r4[e] += __bfloat162float(__float2bfloat16_rn(v[i + e]));
+              for (int e = 0; e < 4; ++e) r4[e] += v[i + e];
               store16(out + i, r4);
             }
           } else {
-            for (int i = 0; i < 32 && n0 + c + i < a.N; ++i) out[i] += __bfloat162float(__float2bfloat16_rn(v[i]));
+            for (int i = 0; i < 32 && n0 + c + i < a.N; ++i) out[i] += v[i];
           }
         }
       }

@@ -146,6 +146,9 @@ class StepContext:
     # the single-token sequences' context lengths (new token included): the longest and their sum
     decode_max_ctx: int = 0
     decode_sum_ctx: int = 0
+    # every sublayer that adds its output product to the stream as a float32 sum in a step of 64 rows does so at any
+    # number of rows (set for scoring; other prompt steps round that product to the activation type before the add)
+    float32_sums: bool = False
     host: Optional["HostBatch"] = None
     profiler: Optional[object] = None          # engine.profiler.OpProfiler while per-op profiling is on
     # a norm handed over between parts (parts.base.NormHandover); set and cleared by the block

@@ -175,6 +175,7 @@ class ModelRunner:
         """Runs the segments' tokens (none of which wants its logits) and returns what ``DecoderModel.body`` does:
         for callers that take the logits of more rows than the logits buffer has, block by block (``score``)."""
         ctx = self.builder.build(segments)
+        ctx.float32_sums = True
         if self.profiler is not None:
             ctx.profiler = self.profiler
             self.profiler.begin("prefill")

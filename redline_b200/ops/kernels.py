@@ -355,6 +355,11 @@ def mid_rows(rows: int, *weights: torch.Tensor) -> bool:
     aligned rows.  ``REDLINE_MID_PRODUCTS=0`` says no (for comparisons)."""
     if rows <= 0 or rows > MID_ROUTED_ROWS or os.environ.get("REDLINE_MID_PRODUCTS", "1") == "0":
         return False
+    return tc_weights(*weights)
+
+
+def tc_weights(*weights: torch.Tensor) -> bool:
+    """Whether gemm_tc and gemm_mid take products over these weights (with activations in rows of a workspace)."""
     return all(w.dtype == torch.bfloat16 and w.is_contiguous() and w.shape[1] % 8 == 0 and w.data_ptr() % 16 == 0
                for w in weights)
 

@@ -85,6 +85,18 @@ class SwiGLUMLP(FeedForward):
         feed-forward, a shared expert for instance, names another)."""
         p, rt = self.params, self.rt
         T = ctx.T
+        act = self._activated(x, ctx, name)
+        out = rt.workspace.get(name + ".out", (rt.max_tokens, p.hidden_size), rt.dtype)[:T]
+        linear(act, self.w_down, out)
+        if self.b_down is not None:
+            kernels.add_bias(out, self.b_down)
+        op_mark(ctx, "down_proj", self.w_down, T)
+        return out
+
+    def _activated(self, x, ctx, name: str) -> torch.Tensor:
+        """act(gate(x)) * up(x)."""
+        p, rt = self.params, self.rt
+        T = ctx.T
         ws = rt.workspace
         act = ws.get(name + ".act", (rt.max_tokens, p.intermediate_size), rt.dtype)[:T]
         tc_epilogue = {"silu": kernels.EPI_SWIGLU, "gelu_tanh": kernels.EPI_GEGLU_TANH,
@@ -108,12 +120,7 @@ class SwiGLUMLP(FeedForward):
             else:
                 kernels.gated_act(gu, act, kernels.ACTIVATIONS[self.params.activation], bias=self.b_gate_up)
         op_mark(ctx, "gate_up+swiglu" if self.silu else "gate_up+act", self.w_gate_up, T)
-        out = ws.get(name + ".out", (rt.max_tokens, p.hidden_size), rt.dtype)[:T]
-        linear(act, self.w_down, out)
-        if self.b_down is not None:
-            kernels.add_bias(out, self.b_down)
-        op_mark(ctx, "down_proj", self.w_down, T)
-        return out
+        return act
 
     def forward_into(self, residual, norm, ctx) -> bool:
         rt = self.rt
@@ -126,6 +133,8 @@ class SwiGLUMLP(FeedForward):
             return self._into_skinny(residual, rms, ctx)
         if kernels.mid_rows(T, self.w_gate_up, self.w_down):
             return self._into_mid(residual, rms, ctx)
+        if ctx.float32_sums and kernels.tc_weights(self.w_gate_up, self.w_down):
+            return self._into_wide(residual, rms, ctx)
         return False
 
     def _into_skinny(self, residual, rms, ctx) -> bool:
@@ -175,4 +184,17 @@ class SwiGLUMLP(FeedForward):
                          hand_out=None if out is None else (out.norm.rms_params()[0], out.xw, out.sums))
         op_mark(ctx, "down_proj+add", self.w_down, T)
         ctx.hand_out = out
+        return True
+
+    def _into_wide(self, residual, rms, ctx) -> bool:
+        """More rows, in steps that keep float32 sums (``ctx.float32_sums``): the down product adds its accumulators
+        to the stream as they are."""
+        rt = self.rt
+        T = ctx.T
+        xn = rt.workspace.get("block.normed", (rt.max_tokens, residual.shape[1]), rt.dtype)[:T]
+        kernels.add_rmsnorm(residual, None, rms[0], xn, rms[1], rows=T)
+        op_mark(ctx, "rmsnorm", nbytes=T * residual.shape[1] * 6.0)
+        act = self._activated(xn, ctx, "ffn")
+        kernels.gemm_tc(act, self.w_down, residual, kernels.EPI_ADD_RESIDUAL)
+        op_mark(ctx, "down_proj+add", self.w_down, T)
         return True

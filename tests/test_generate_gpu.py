@@ -148,6 +148,31 @@ def test_score_in_portions(models):
     assert eng.runner.cache.num_open() == 0
 
 
+@pytest.mark.parametrize("T", [65, 130, 256])
+def test_scored_portions_add_float32_sums(T, tmp_path):
+    """The stream behind one layer's two sublayers is the embedding plus both output products of the 16-bit activations
+    that the layer left, summed in float32 (bound: 2^-16 of the products' absolute terms; a product rounded to bfloat16
+    before the add is off by up to 2^-9 of itself)."""
+    from redline_b200.engine.batch import Segment
+    from redline_b200.engine.engine import Engine
+    cfg = dict(C.TINY_A, num_hidden_layers=1)
+    d, w = make_model(tmp_path, cfg, seed=46, sharpen=5.0)
+    eng = Engine(d, dtype="bfloat16", max_num_seqs=2, max_num_batched_tokens=256, max_seq_len=512, kv_cache_tokens=512)
+    run = eng.runner
+    toks = random_tokens(512, T, 9)
+    rc = run.open("s")
+    assert run.cache.reserve(rc, T)
+    residual, pending = run.run_body([Segment(rc, toks, 0)])
+    assert pending is None
+    attn, act = (run.rt.workspace.get(n, (256, x.shape[1]), torch.bfloat16)[:T].double().cpu() for n, x in (
+        ("attn.out", w["model.layers.0.self_attn.o_proj.weight"]), ("ffn.act", w["model.layers.0.mlp.down_proj.weight"])))
+    o, down = w["model.layers.0.self_attn.o_proj.weight"].double(), w["model.layers.0.mlp.down_proj.weight"].double()
+    want = w["model.embed_tokens.weight"].double()[toks] + attn @ o.T + act @ down.T
+    bound = 2.0 ** -16 * (attn.abs() @ o.abs().T + act.abs() @ down.abs().T) + 2.0 ** -22 * want.abs()
+    assert ((residual.double().cpu() - want).abs() <= bound).all()
+    run.close("s")
+
+
 def test_command_line(models, tmp_path):
     d, w = models["tiny_a"]
     p = random_tokens(512, 9, 3)

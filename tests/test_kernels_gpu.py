@@ -902,6 +902,20 @@ def test_gemm_tc_epilogues(M, N, K, tile_n):
     assert int(status.item()) == 0                   # no wait inside the kernel ran out
 
 
+@pytest.mark.parametrize("tile_n", [128, 256, 512])
+@pytest.mark.parametrize("M,N,K", [(65, 331, 200), (130, 200, 72), (300, 1000, 384)])
+def test_gemm_tc_adds_its_accumulators(M, N, K, tile_n):
+    """residual += product with the product as it was accumulated (float32 sums of K terms and one add)."""
+    g = torch.Generator(device="cuda").manual_seed(M + N + K)
+    x = torch.randn(M, K, device=DEV, generator=g).to(torch.bfloat16)
+    w = (torch.randn(N, K, device=DEV, generator=g) * 0.05).to(torch.bfloat16)
+    res = torch.randn(M, N, device=DEV, generator=g)
+    want = res.double() + x.double() @ w.double().T
+    kernels.gemm_tc(x, w, res, kernels.EPI_ADD_RESIDUAL, tile_n)
+    assert int(kernels.tc_status(x.device).item()) == 0
+    close(res, want, 2e-5)
+
+
 def test_gemm_tc_refuses_what_it_cannot_do():
     x = torch.zeros(4, 20, device=DEV, dtype=torch.bfloat16)
     w = torch.zeros(32, 20, device=DEV, dtype=torch.bfloat16)
