@@ -60,11 +60,6 @@ class _InFlight:
     record: StepRecord
 
 
-# The most that ``score`` allocates for logits beside the engine's own buffer (512 rows of a vocabulary of 128,256: the
-# head is then bound by its products and not by reading its table for every 64 rows).
-SCORE_LOGITS_BYTES = 256 << 20
-
-
 def make_output(seq: Sequence) -> Dict[str, Any]:
     return {
         "id": seq.id,
@@ -323,23 +318,17 @@ class Engine:
             n = len(tokens) - 1
             chunk = min(self.cfg.max_num_batched_tokens, n)
             logits = self.runner.logits
-            rows = min(chunk, SCORE_LOGITS_BYTES // (4 * self.vocab_size))
+            rows = min(chunk, self.runner.score_block_rows())
             if rows > logits.shape[0]:
                 try:
                     logits = torch.empty((rows, self.vocab_size), dtype=torch.float32, device=self.runner.device)
                 except torch.OutOfMemoryError:
                     pass
-            rows = logits.shape[0]
             target = torch.tensor(tokens[1:], dtype=torch.int32).to(self.runner.device)
             lp = torch.empty(n, dtype=torch.float32, device=self.runner.device)
-            from ..ops import kernels
             for s in range(0, n, chunk):
                 m = min(chunk, n - s)
-                residual, pending = self.runner.run_body([Segment(rc, tokens[s:s + m], s)])
-                for r in range(0, m, rows):
-                    k = min(rows, m - r)
-                    block = self.runner.model.head_over(residual[r:r + k], None if pending is None else pending[r:r + k], logits)
-                    kernels.gather_logprob(block, k, target[s + r:s + r + k], lp[s + r:s + r + k])
+                self.runner.score(Segment(rc, tokens[s:s + m], s), target[s:s + m], lp[s:s + m], logits)
             out = lp.tolist()
         finally:
             self.runner.close(key)

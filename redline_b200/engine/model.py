@@ -213,10 +213,14 @@ class DecoderModel:
             op_mark(ctx, "lm_head", head_w, R, nbytes=R * logits.shape[1] * 2.0)     # (the logits are float32: 2 more bytes each)
         return logits[:R]
 
-    def head_over(self, residual: torch.Tensor, pending: Optional[torch.Tensor], logits: torch.Tensor) -> torch.Tensor:
-        """Logits of every row that ``body`` left in ``residual`` / ``pending`` (at most as many as ``logits`` has)."""
+    def head_over(self, ctx, residual: torch.Tensor, pending: Optional[torch.Tensor], logits: torch.Tensor,
+                  most: int) -> torch.Tensor:
+        """Logits of every row of ``residual`` / ``pending``, a block of what ``body`` left (no more rows than ``logits``
+        has, nor than ``most``, the rows that the buffer of normed rows is kept for)."""
         rows = residual.shape[0]
-        xr = self.rt.workspace.get("head.rows", (logits.shape[0], self.spec.hidden_size), self.rt.dtype)[:rows]
+        xr = self.rt.workspace.get("head.rows", (most, self.spec.hidden_size), self.rt.dtype)[:rows]
         self.final_norm.add_norm(residual, pending, xr, rows=rows)
+        op_mark(ctx, "final_norm", nbytes=rows * self.spec.hidden_size * 6.0)
         self.head.forward(xr, rows, logits)
+        op_mark(ctx, "lm_head", getattr(self.head, "weight", None), rows, nbytes=rows * logits.shape[1] * 2.0)
         return logits[:rows]

@@ -31,6 +31,9 @@ from .model import DecoderModel
 
 GRAPH_BUCKETS = (1, 2, 4, 8, 12, 16, 24, 32, 48, 64, 96, 128, 160, 192, 256, 384, 512)
 GRAPH_MAX_ROWS = 1024          # no graph is captured for more rows than this
+# The most that ``score`` allocates for logits beside the engine's own buffer (512 rows of a vocabulary of 128,256: the
+# head is then bound by its products and not by reading its table for every 64 rows).
+SCORE_LOGITS_BYTES = 256 << 20
 STATUS_MESSAGES = {1: "a token id outside the vocabulary", 2: "a position beyond the rotary table",
                    4: "a cache slot beyond the pool"}
 
@@ -171,21 +174,35 @@ class ModelRunner:
                 self.profiler.end()
         return self.logits[:ctx.R], ctx
 
-    def run_body(self, segments: Sequence[Segment]) -> Tuple[torch.Tensor, Optional[torch.Tensor]]:
-        """Runs the segments' tokens (none of which wants its logits) and returns what ``DecoderModel.body`` does:
-        for callers that take the logits of more rows than the logits buffer has, block by block (``score``)."""
-        ctx = self.builder.build(segments)
+    def score_block_rows(self) -> int:
+        """Rows of logits that ``score`` holds at once beside the engine's own buffer: SCORE_LOGITS_BYTES of them, in
+        whole 128-row tiles of the head's product."""
+        most = SCORE_LOGITS_BYTES // (4 * self.vocab_size)
+        if most >= 128:
+            most -= most % 128
+        return min(self.cfg.max_num_batched_tokens, most)
+
+    def score(self, segment: Segment, target: torch.Tensor, out: torch.Tensor, logits: torch.Tensor) -> None:
+        """Runs the segment's tokens as one step and writes log p(target[i] | tokens up to i) to out[i]; the head
+        runs over blocks of as many rows as ``logits`` has.  The sublayers' sums are float32 (see StepContext)."""
+        ctx = self.builder.build([segment])
         ctx.float32_sums = True
         if self.profiler is not None:
             ctx.profiler = self.profiler
             self.profiler.begin("prefill")
         before = kernels.LAUNCHES
-        out = self.model.body(ctx, self._caches, self._states)
+        residual, pending = self.model.body(ctx, self._caches, self._states)
+        rows, most = logits.shape[0], max(self.max_rows, self.score_block_rows())
+        for r in range(0, ctx.T, rows):
+            k = min(rows, ctx.T - r)
+            block = self.model.head_over(ctx, residual[r:r + k], None if pending is None else pending[r:r + k], logits, most)
+            kernels.gather_logprob(block, k, target[r:r + k], out[r:r + k])
+            if ctx.profiler is not None:
+                ctx.profiler.mark("logprobs", k * self.vocab_size * 4.0, 0.0)
         self.num_eager_steps += 1
         self.num_kernel_launches += kernels.LAUNCHES - before
         if self.profiler is not None:
             self.profiler.end()
-        return out
 
     def _forward(self, ctx: StepContext, sample: bool, resolve: bool) -> None:
         if resolve:

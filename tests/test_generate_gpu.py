@@ -162,7 +162,9 @@ def test_scored_portions_add_float32_sums(T, tmp_path):
     toks = random_tokens(512, T, 9)
     rc = run.open("s")
     assert run.cache.reserve(rc, T)
-    residual, pending = run.run_body([Segment(rc, toks, 0)])
+    ctx = run.builder.build([Segment(rc, toks, 0)])
+    ctx.float32_sums = True
+    residual, pending = run.model.body(ctx, run._caches, run._states)
     assert pending is None
     attn, act = (run.rt.workspace.get(n, (256, x.shape[1]), torch.bfloat16)[:T].double().cpu() for n, x in (
         ("attn.out", w["model.layers.0.self_attn.o_proj.weight"]), ("ffn.act", w["model.layers.0.mlp.down_proj.weight"])))
@@ -171,6 +173,26 @@ def test_scored_portions_add_float32_sums(T, tmp_path):
     bound = 2.0 ** -16 * (attn.abs() @ o.abs().T + act.abs() @ down.abs().T) + 2.0 ** -22 * want.abs()
     assert ((residual.double().cpu() - want).abs() <= bound).all()
     run.close("s")
+
+
+def test_scoring_is_counted_and_profiled(models, monkeypatch):
+    """Every launch of a scored text is in the runner's count, and the per-op profile has the head of every block."""
+    from redline_b200.engine import runner
+    from redline_b200.engine.engine import Engine
+    from redline_b200.ops import kernels
+    monkeypatch.setattr(runner, "SCORE_LOGITS_BYTES", 24 * 512 * 4)
+    d, _ = models["tiny_a"]
+    eng = Engine(d, dtype="bfloat16", max_num_seqs=2, max_num_batched_tokens=64, max_logit_rows=16, max_seq_len=256,
+                 kv_cache_tokens=512)
+    toks = random_tokens(512, 150, 8)
+    eng.score(toks)
+    before, counted = kernels.LAUNCHES, eng.runner.num_kernel_launches
+    eng.runner.set_op_profiling(True)
+    eng.score(toks)
+    assert eng.runner.num_kernel_launches - counted == kernels.LAUNCHES - before
+    calls = {r["op"]: r["calls_per_pass"] for r in eng.runner.profiler.report()}
+    blocks = 3 + 3 + 1               # three passes: portions of 64, 64 and 21 tokens in blocks of 24 rows
+    assert all(abs(3 * calls["prefill/" + op] - blocks) < 1e-6 for op in ("final_norm", "lm_head", "logprobs"))
 
 
 def test_command_line(models, tmp_path):
