@@ -78,8 +78,11 @@ class Workspace:
             for k in [k for k in self._views if k[0] == name and k[2] is dtype]:
                 del self._views[k]              # (views of the buffer that this one replaces)
         view = buf[:n].view(shape)
-        if len(self._views) < 1024:             # (shapes are a part's widest: a model has some dozens of them)
-            self._views[(name, shape, dtype)] = view
+        # (a model asks for some dozens of shapes in every step, and now and then for one that depends on the step;
+        # the oldest goes when there are many: a step's own is back after its next request)
+        if len(self._views) >= 1024:
+            del self._views[next(iter(self._views))]
+        self._views[(name, shape, dtype)] = view
         return view
 
     def nbytes(self) -> int:
