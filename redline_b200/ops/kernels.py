@@ -49,11 +49,14 @@ def _fn(lib: ctypes.CDLL, name: str, argtypes):
 # stay out of torch's Python layers: a stream handle by ``torch.cuda.current_stream()`` alone was 7 us of the 20 us
 # that a launch took, pointers wrapped in c_void_p another 2 (plain integers do as well).  A prompt of 333 tokens
 # went from 3.06 to 1.98 ms with them and the workspace's kept views.
-_raw_stream = torch._C._cuda_getCurrentRawStream
-_device_index = torch._C._cuda_getDevice
+# (A torch without CUDA has neither function: the module still imports there, and a launch says why it cannot be.)
+_raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+_device_index = getattr(torch._C, "_cuda_getDevice", None)
 
 
 def _stream() -> int:
+    if _raw_stream is None or _device_index is None:
+        raise KernelError("redline_b200 kernels need a torch that was built with CUDA")
     return _raw_stream(_device_index())
 
 
