@@ -148,6 +148,55 @@ def test_score_in_portions(models):
     assert eng.runner.cache.num_open() == 0
 
 
+def log_probs(logits, toks):
+    lp = torch.log_softmax(torch.as_tensor(logits).double(), -1)
+    return np.array([float(lp[i, toks[i + 1]]) for i in range(len(toks) - 1)])
+
+
+@pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
+@pytest.mark.parametrize("rows,own", [(24, 16), (0, 40)])
+@pytest.mark.parametrize("n,batched", [(154, 64), (129, 64), (218, 200), (26, 64)])
+def test_score_over_several_blocks(n, batched, rows, own, dtype, models, monkeypatch):
+    """A portion whose logits come in several blocks, of a buffer of 24 rows and of the engine's own (nothing else is
+    allocated): ragged last blocks, last blocks of one row, last portions of one token; the stream's last addend is
+    pending (float32) or added already (bfloat16)."""
+    from redline_b200.engine import runner
+    from redline_b200.engine.engine import Engine
+    monkeypatch.setattr(runner, "SCORE_LOGITS_BYTES", rows * 512 * 4)
+    d, w = models["tiny_a"]
+    eng = Engine(d, dtype=dtype, max_num_seqs=2, max_num_batched_tokens=batched, max_logit_rows=own, max_seq_len=256,
+                 kv_cache_tokens=512)
+    toks = random_tokens(512, n, 80 + n)
+    got = np.array(eng.score(toks))
+    diff = np.abs(got - log_probs(oracle_logits(C.TINY_A, w, toks), toks))
+    # (bfloat16: the reference's bounds for its half-precision engine, see gpu_utils)
+    assert diff.max() < 1e-3 if dtype == "float32" else diff.mean() < 0.03 and diff.max() < 0.3
+    assert eng.runner.cache.num_open() == 0
+
+
+@pytest.mark.parametrize("design,name,dtype", [("vizotar", "mix", "float32"), ("vizotar", "calm", "bfloat16"),
+                                               ("kapitar", "mix", "float32"), ("kapitar", "plain", "bfloat16")])
+def test_score_of_models_with_states_and_streams(design, name, dtype, tmp_path, monkeypatch):
+    """Several residual streams, mixers that carry a state from portion to portion: the log-probabilities of the logits
+    that ``step_tokens`` gives for the same portions (float32 sums of the head in another order: 1e-3)."""
+    import importlib
+    from redline_b200.engine import runner
+    utils, configs = importlib.import_module(design + "_utils"), importlib.import_module(design + "_configs")
+    cfg = configs.ALL[name]
+    monkeypatch.setattr(runner, "SCORE_LOGITS_BYTES", 24 * cfg["vocab"] * 4)
+    d, _ = utils.make_model(tmp_path, cfg, seed=5)
+    eng = utils.engine_for(d, dtype, max_num_batched_tokens=64, max_logit_rows=64)
+    toks = random_tokens(cfg["vocab"], 154, 11)
+    logits = []
+    for s in range(0, 153, 64):
+        part = toks[s:min(s + 64, 153)]
+        logits.append(eng.step_tokens([("w", part, list(range(len(part))))]).cpu())
+    eng.close_request("w")
+    eng.runner.max_rows, eng.runner.logits = 16, eng.runner.logits[:16]          # as if that were all the engine keeps
+    got = np.array(eng.score(toks))
+    assert np.abs(got - log_probs(torch.cat(logits), toks)).max() < 1e-3
+
+
 @pytest.mark.parametrize("T", [65, 130, 256])
 def test_scored_portions_add_float32_sums(T, tmp_path):
     """The stream behind one layer's two sublayers is the embedding plus both output products of the 16-bit activations
