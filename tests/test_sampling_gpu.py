@@ -122,6 +122,21 @@ def test_draw_over_a_cluster_equals_the_plain_restatement(V, ld, T, k, p):
     assert np.abs(lp - want.numpy()).max() < 1e-4
 
 
+@pytest.mark.parametrize("T,k,p", [(1.0, 0, 0.95), (1.4, 200, 0.9), (3.0, 40000, 0.8)])
+def test_draw_at_a_served_vocabulary(T, k, p):
+    """128,256 logits, 64 KB of a row to a CTA (more than a kernel has without asking): tokens drawn from flat and from
+    peaked rows, which are not the arg max."""
+    V = 128256
+    rng = np.random.RandomState(int(10 * T))
+    l = (rng.randn(4, V) * np.array([[0.1], [1.0], [2.5], [1.0]])).astype(np.float32)
+    l[3] = np.round(4 * l[3]) / 4                          # ties at every threshold
+    tok, lp = run(torch.from_numpy(l).to(DEV), T, k, p, 987654321, np.arange(4) + 11)
+    want = [P.gumbel_draw(l[r], T, k, p, 987654321, r + 11) for r in range(4)]
+    assert tok.tolist() == want and sum(int(l[r].argmax()) != want[r] for r in range(4)) >= 3
+    full = torch.log_softmax(torch.from_numpy(l).double(), -1)[torch.arange(4), torch.tensor(want)]
+    assert np.abs(lp - full.numpy()).max() < 1e-4
+
+
 @pytest.mark.parametrize("two_stage", [False, True])
 @pytest.mark.parametrize("V", [1, 331, 8191, 8192, 20001, 128256])
 def test_rows_without_a_best_logit(V, two_stage):
