@@ -45,6 +45,17 @@ __device__ __forceinline__ void copy16(void* dst, const void* src, bool in) {
   const int n = in ? 16 : 0;
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(src), "r"(n) : "memory");
 }
+// The same with 4 or 8 bytes (aligned to as many).
+template <int BYTES>
+__device__ __forceinline__ void copy_piece(void* dst, const void* src, bool in) {
+  if constexpr (BYTES == 16) {
+    copy16(dst, src, in);
+  } else {
+    const uint32_t d = static_cast<uint32_t>(__cvta_generic_to_shared(dst));
+    const int n = in ? BYTES : 0;
+    asm volatile("cp.async.ca.shared.global [%0], [%1], %2, %3;" ::"r"(d), "l"(src), "n"(BYTES), "r"(n) : "memory");
+  }
+}
 __device__ __forceinline__ void commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 template <int N>
 __device__ __forceinline__ void wait_group() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
@@ -161,8 +172,13 @@ simt_few_kernel(const float* __restrict__ w, const float* x, float* y, int M, in
 //
 // A block computes 64 x 64 outputs; its four groups of 64 threads take a quarter of K each, 8 x 8 outputs a thread.
 // Shared memory holds rows as they are (16 k of a row, 20 floats apart: conflict-free 16-byte reads along k, and
-// the pairs of a packed fma lie side by side).  The quarters meet in shared memory at the end.  kAsync: float
-// operands on 16-byte boundaries, copied through a ring of four stages; otherwise loads entry by entry.
+// the pairs of a packed fma lie side by side; bfloat16 rows stay bfloat16 and are widened when they are read).  The
+// quarters meet in shared memory at the end.  P: the entries of an asynchronous copy into the ring of four stages, 4
+// where every four k of both operands start on a boundary of their size, else 1 for two float operands; 0: loads
+// entry by entry (a bfloat16 entry is too small to copy).
+// Mixed types took the loads of P = 0, one after the other, in every case at first: 224 to 270 us for one row, 330 to
+// 416 for 64, 2,000 for 2,048 at N 2048 K 2048 (the kernel of 64 x 64 tiles before: 135 to 150, 143 to 159, 690); with
+// copies 29 to 33, 72 to 75, 502 to 521; with the loads of P = 0 asked for together (K 2045, 2046) 55, 91 to 96, 566 to 594.
 // Bound: the FFMA pipe and the shared-memory reads, one after the other (2,048 cycles each a stage; 31 of 74 TFLOP/s).
 // Plain instead of packed multiply-adds, or 8 x 4 outputs a thread on twice the warps, come out the same.
 // The last tile of rows is often short of 64 (two prompts of 100 tokens leave 8): it runs with as many eights of rows as
@@ -176,7 +192,15 @@ constexpr int kTlStageFloats = kQuarters * kTlGroupFloats;
 constexpr int kTlSmem = kTlStages * kTlStageFloats * 4;
 static_assert(kTlStages * kTlStageFloats >= (kQuarters - 1) * kTile * kTile, "the quarters' sums fit the ring");
 
-template <typename TA, typename TW, typename TC, bool kAsync>
+// Four neighbouring k of a row in shared memory, as the two pairs of a packed multiply-add.
+__device__ __forceinline__ ulonglong2 four(const float* p) { return *reinterpret_cast<const ulonglong2*>(p); }
+__device__ __forceinline__ ulonglong2 four(const bf16* p) {
+  const uint2 u = *reinterpret_cast<const uint2*>(p);
+  auto pair = [](uint32_t v) { return static_cast<unsigned long long>(v & 0xffff0000u) << 32 | (v << 16); };
+  return make_ulonglong2(pair(u.x), pair(u.y));
+}
+
+template <typename TA, typename TW, typename TC, int P>
 __global__ void __launch_bounds__(kTlThreads, 1)
 simt_tile_kernel(const TA* x, const TW* __restrict__ w, TC* y, int M, int N, int K, int ldx, int ldy) {
   pdl_launch();
@@ -190,27 +214,38 @@ simt_tile_kernel(const TA* x, const TW* __restrict__ w, TC* y, int M, int N, int
 
   auto ask = [&](int s) {
     float* st = sm + (s % kTlStages) * kTlStageFloats + g * kTlGroupFloats;
-    if constexpr (kAsync) {
+    TA* xs = reinterpret_cast<TA*>(st);
+    TW* ws = reinterpret_cast<TW*>(st + kTile * kTlPitch);
+    if constexpr (P > 0) {
+      constexpr int kPieces = kTlK / P, kRowsApart = kTlGroup / kPieces;
+      const int at = t % kPieces * P, off = s * kTlK + at, k = g * ql + off;
+      const bool in = off < ql && k < K;
 #pragma unroll
-      for (int j = 0; j < 2 * kTile * 4 / kTlGroup; ++j) {
-        const int c = j * kTlGroup + t, row = c >> 2, piece = c & 3;           // rows 0..63 of x, then of the weights
-        const int off = s * kTlK + piece * 4, k = g * ql + off;
-        const bool is_x = j < kTile * 4 / kTlGroup;
-        const int r = is_x ? m0 + row : n0 + row - kTile;
-        const bool in = r < (is_x ? M : N) && off < ql && k < K;
-        const void* src = is_x ? static_cast<const void*>(x + static_cast<size_t>(r) * ldx + k)
-                               : static_cast<const void*>(w + static_cast<size_t>(r) * K + k);
-        copy16(st + row * kTlPitch + piece * 4, in ? src : static_cast<const void*>(w), in);
+      for (int j = 0; j < kTile / kRowsApart; ++j) {
+        const int row = j * kRowsApart + t / kPieces;
+        const bool xin = in && m0 + row < M, win = in && n0 + row < N;
+        copy_piece<P * sizeof(TA)>(xs + row * kTlPitch + at, xin ? x + static_cast<size_t>(m0 + row) * ldx + k : x, xin);
+        copy_piece<P * sizeof(TW)>(ws + row * kTlPitch + at, win ? w + static_cast<size_t>(n0 + row) * K + k : w, win);
       }
     } else {
-      for (int c = t; c < 2 * kTile * kTlK; c += kTlGroup) {
-        const int row = c / kTlK, off = s * kTlK + c % kTlK, k = g * ql + off;
-        const bool is_x = row < kTile;
-        const int r = is_x ? m0 + row : n0 + row - kTile;
-        float v = 0.f;
-        if (r < (is_x ? M : N) && off < ql && k < K)
-          v = is_x ? to_float(x[static_cast<size_t>(r) * ldx + k]) : to_float(w[static_cast<size_t>(r) * K + k]);
-        st[row * kTlPitch + c % kTlK] = v;
+      // (a thread has one k of every fourth row; all its loads, from places inside the operands, are on their way
+      // before the first is stored)
+      constexpr int kRowsApart = kTlGroup / kTlK, kLoads = kTile / kRowsApart;
+      const int off = s * kTlK + t % kTlK, k = g * ql + off, kc = min(k, K - 1);
+      const bool in = off < ql && k < K;
+      TA xv[kLoads];
+      TW wv[kLoads];
+#pragma unroll
+      for (int j = 0; j < kLoads; ++j) {
+        const int row = j * kRowsApart + t / kTlK;
+        xv[j] = x[static_cast<size_t>(min(m0 + row, M - 1)) * ldx + kc];
+        wv[j] = w[static_cast<size_t>(min(n0 + row, N - 1)) * K + kc];
+      }
+#pragma unroll
+      for (int j = 0; j < kLoads; ++j) {
+        const int row = j * kRowsApart + t / kTlK;
+        xs[row * kTlPitch + t % kTlK] = in && m0 + row < M ? xv[j] : from_float<TA>(0.f);
+        ws[row * kTlPitch + t % kTlK] = in && n0 + row < N ? wv[j] : from_float<TW>(0.f);
       }
     }
   };
@@ -235,8 +270,10 @@ simt_tile_kernel(const TA* x, const TW* __restrict__ w, TC* y, int M, int N, int
       if (s + kTlStages - 1 < steps) ask(s + kTlStages - 1);
       commit();
       const float* st = sm + (s % kTlStages) * kTlStageFloats + g * kTlGroupFloats;
-      auto x4 = [&](int i, int p) { return *reinterpret_cast<const ulonglong2*>(st + (i * 8 + ty) * kTlPitch + p * 4); };
-      auto w4 = [&](int j, int p) { return *reinterpret_cast<const ulonglong2*>(st + (kTile + j * kTlCols + tx) * kTlPitch + p * 4); };
+      const TA* xs = reinterpret_cast<const TA*>(st);
+      const TW* ws = reinterpret_cast<const TW*>(st + kTile * kTlPitch);
+      auto x4 = [&](int i, int p) { return four(xs + (i * 8 + ty) * kTlPitch + p * 4); };
+      auto w4 = [&](int j, int p) { return four(ws + (j * kTlCols + tx) * kTlPitch + p * 4); };
       ulonglong2 a[2][MI], b[2];
 #pragma unroll
       for (int i = 0; i < MI; ++i) a[0][i] = x4(i, 0);
@@ -298,13 +335,27 @@ int raise_smem(int bytes) {
   return static_cast<int>(e);
 }
 
-template <typename TA, typename TW, typename TC, bool kAsync>
+template <typename TA, typename TW, typename TC, int P>
 int launch_tile(const void* x, const void* w, void* y, int M, int N, int K, int ldx, int ldy, cudaStream_t stream) {
-  if (const int e = raise_smem<simt_tile_kernel<TA, TW, TC, kAsync>>(kTlSmem)) return e;
+  if (const int e = raise_smem<simt_tile_kernel<TA, TW, TC, P>>(kTlSmem)) return e;
   dim3 grid((N + kTile - 1) / kTile, (M + kTile - 1) / kTile);
-  launch_kernel(simt_tile_kernel<TA, TW, TC, kAsync>, grid, dim3(kTlThreads), kTlSmem, stream, static_cast<const TA*>(x),
+  launch_kernel(simt_tile_kernel<TA, TW, TC, P>, grid, dim3(kTlThreads), kTlSmem, stream, static_cast<const TA*>(x),
                 static_cast<const TW*>(w), static_cast<TC*>(y), M, N, K, ldx, ldy);
   return static_cast<int>(cudaGetLastError());
+}
+
+// Whether every four k of both operands lie on a boundary of their size.
+template <typename TA, typename TW>
+bool in_fours(const void* x, const void* w, int K, int ldx) {
+  return K % 4 == 0 && ldx % 4 == 0 && reinterpret_cast<uintptr_t>(x) % (4 * sizeof(TA)) == 0 &&
+         reinterpret_cast<uintptr_t>(w) % (4 * sizeof(TW)) == 0;
+}
+
+template <typename TA, typename TW, typename TC>
+int launch_tiles(const void* x, const void* w, void* y, int M, int N, int K, int ldx, int ldy, cudaStream_t stream) {
+  if (in_fours<TA, TW>(x, w, K, ldx)) return launch_tile<TA, TW, TC, 4>(x, w, y, M, N, K, ldx, ldy, stream);
+  constexpr int kRest = sizeof(TA) == 4 && sizeof(TW) == 4 ? 1 : 0;          // (the smallest asynchronous copy is 4 bytes)
+  return launch_tile<TA, TW, TC, kRest>(x, w, y, M, N, K, ldx, ldy, stream);
 }
 
 template <int MR, int NPT, int MG, int STAGES>
@@ -325,11 +376,9 @@ bool few_rows(int M, int N) {
 }
 
 int launch_f32(const void* xv, const void* wv, void* yv, int M, int N, int K, int ldx, int ldy, cudaStream_t stream) {
-  const bool aligned = K % 4 == 0 && ldx % 4 == 0 && reinterpret_cast<uintptr_t>(xv) % 16 == 0 &&
-                       reinterpret_cast<uintptr_t>(wv) % 16 == 0;
-  if (!aligned) return launch_tile<float, float, float, false>(xv, wv, yv, M, N, K, ldx, ldy, stream);
   const long long chunks = (static_cast<long long>(M) + 15) / 16;
-  if (!few_rows(M, N) || chunks > 65535) return launch_tile<float, float, float, true>(xv, wv, yv, M, N, K, ldx, ldy, stream);
+  if (!in_fours<float, float>(xv, wv, K, ldx) || !few_rows(M, N) || chunks > 65535)
+    return launch_tiles<float, float, float>(xv, wv, yv, M, N, K, ldx, ldy, stream);
   const float *x = static_cast<const float*>(xv), *w = static_cast<const float*>(wv);
   float* y = static_cast<float*>(yv);
   if (M == 1) return launch_few<1, 1, 1, 6>(x, w, y, M, N, K, ldx, ldy, stream);
@@ -352,13 +401,13 @@ int rl_gemm_tn_simt(const void* x, int x_dtype, const void* w, int w_dtype, void
   const int code = x_dtype * 4 + w_dtype * 2 + y_dtype;
   switch (code) {
     case 0: return launch_f32(x, w, y, M, N, K, ldx, ldy, stream);
-    case 1: return launch_tile<float, float, bf16, false>(x, w, y, M, N, K, ldx, ldy, stream);
-    case 2: return launch_tile<float, bf16, float, false>(x, w, y, M, N, K, ldx, ldy, stream);
-    case 3: return launch_tile<float, bf16, bf16, false>(x, w, y, M, N, K, ldx, ldy, stream);
-    case 4: return launch_tile<bf16, float, float, false>(x, w, y, M, N, K, ldx, ldy, stream);
-    case 5: return launch_tile<bf16, float, bf16, false>(x, w, y, M, N, K, ldx, ldy, stream);
-    case 6: return launch_tile<bf16, bf16, float, false>(x, w, y, M, N, K, ldx, ldy, stream);
-    case 7: return launch_tile<bf16, bf16, bf16, false>(x, w, y, M, N, K, ldx, ldy, stream);
+    case 1: return launch_tiles<float, float, bf16>(x, w, y, M, N, K, ldx, ldy, stream);
+    case 2: return launch_tiles<float, bf16, float>(x, w, y, M, N, K, ldx, ldy, stream);
+    case 3: return launch_tiles<float, bf16, bf16>(x, w, y, M, N, K, ldx, ldy, stream);
+    case 4: return launch_tiles<bf16, float, float>(x, w, y, M, N, K, ldx, ldy, stream);
+    case 5: return launch_tiles<bf16, float, bf16>(x, w, y, M, N, K, ldx, ldy, stream);
+    case 6: return launch_tiles<bf16, bf16, float>(x, w, y, M, N, K, ldx, ldy, stream);
+    case 7: return launch_tiles<bf16, bf16, bf16>(x, w, y, M, N, K, ldx, ldy, stream);
   }
   return static_cast<int>(cudaErrorInvalidValue);
 }

@@ -113,6 +113,26 @@ def test_gemm_simt_one_order_of_sums(N, K, ldx):
         assert torch.equal(last, y[M - 1:M, :N]), M
 
 
+@pytest.mark.parametrize("off", [0, 1, 2, 4])
+@pytest.mark.parametrize("K", [4, 36, 131, 134, 516])
+@pytest.mark.parametrize("tx,tw", [("float32", "float32"), ("bfloat16", "float32"), ("float32", "bfloat16"), ("bfloat16", "bfloat16")])
+def test_gemm_simt_operands_off_their_boundaries(tx, tw, K, off):
+    """Copies of four k, of one, and plain loads, by the operands' types and where they start: rows of x that start
+    ``off`` entries into a longer row, K that is no multiple of four.  Float64 within the rounding of ordered sums, and a
+    row's bits the same beside 199 other rows, beside none, and off its boundaries or on them."""
+    N = 70
+    full = torch.randn(200, K + 8, device=DEV).to(DT[tx])
+    x, w = full[:, off:off + K], torch.randn(N, K, device=DEV).to(DT[tw])
+    y, one, whole = (torch.empty(m, N, device=DEV) for m in (200, 1, 200))
+    kernels.gemm_tn_simt(x, w, y)
+    kernels.gemm_tn_simt(x[131:132], w, one)
+    kernels.gemm_tn_simt(x.contiguous(), w, whole)
+    want = x.double() @ w.double().T
+    bound = (x.double().abs() @ w.double().abs().T) * (K / 8 + 8) * 2.0 ** -24
+    assert ((y.double() - want).abs() <= bound).all()
+    assert torch.equal(y[131:132], one) and torch.equal(y, whole)
+
+
 @pytest.mark.parametrize("M,N,K", [(1, 3072, 2048), (8, 1000, 384), (200, 704, 256), (64, 331, 200)])
 def test_linear_bfloat16(M, N, K):
     x = torch.randn(M, K, device=DEV).to(torch.bfloat16)
