@@ -188,10 +188,12 @@ class GQAttention(Mixer):
         return True
 
     def decode_variant(self, ctx) -> int:
-        """4 where the decode kernel of one cluster per (sequence, kv head) is expected to be the fastest (few
-        sequences of similar length), else 0 (the kernels choose among themselves)."""
+        """4 where the decode kernel of one cluster per (sequence, kv head) is expected to be the fastest
+        (kernels.attn_decode_rows_pays) and takes the layer (groups of at most 16 heads), else 0 (the kernels choose among
+        themselves)."""
         p, rt = self.params, self.rt
-        if rt.dtype != torch.bfloat16 or ctx.num_decode <= 0 or os.environ.get("REDLINE_DECODE_ROWS", "1") == "0":
+        if (rt.dtype != torch.bfloat16 or ctx.num_decode <= 0 or p.num_heads > 16 * p.num_kv_heads
+                or os.environ.get("REDLINE_DECODE_ROWS", "1") == "0"):
             return 0
         # (the layers of a model mostly ask the same question: the step's context keeps the answers)
         memo = ctx.__dict__.setdefault("_decode_variants", {})

@@ -148,6 +148,18 @@ def test_score_in_portions(models):
     assert eng.runner.cache.num_open() == 0
 
 
+@pytest.mark.parametrize("heads,head_dim", [(32, 64), (17, 128)])
+def test_more_heads_to_a_kv_head_than_clusters_take(heads, head_dim, tmp_path):
+    """Groups of more than 16 heads, which the decode kernel of a cluster per row refuses: the layer runs another one."""
+    from redline_b200.runtime import Engine
+    cfg = dict(C.TINY_A, num_attention_heads=heads, num_key_value_heads=1, head_dim=head_dim)
+    d, w = make_model(tmp_path, cfg, seed=47, sharpen=5.0)
+    eng = Engine(d, dtype="bfloat16", max_seqs=4, max_batched_tokens=64, max_seq_len=256, kv_cache_tokens=512)
+    p = random_tokens(512, 40, 3)
+    out = eng.generate([p], max_new_tokens=6, ignore_eos=True)[0]["output_ids"]
+    check_greedy(cfg, w, p, out, 0.1)
+
+
 def log_probs(logits, toks):
     lp = torch.log_softmax(torch.as_tensor(logits).double(), -1)
     return np.array([float(lp[i, toks[i + 1]]) for i in range(len(toks) - 1)])
