@@ -1413,8 +1413,8 @@ int rl_attn_tile_rows() { return 4 * kBQ; }
 // 64 or 128, at most 16 heads per group, pages of 16 to 128 keys, at most 512 items), else the
 // one-partition-per-CTA tensor-core kernel, else the CUDA-core kernel; 1 = the CUDA-core kernel;
 // 2 = the one-partition-per-CTA tensor-core kernel or an error; 3 = the streaming kernel or an error;
-// 4 = one cluster per (item, kv head) (decode_rows.cuh: for few rows of similar length) or an error: when the
-// launch has more rows than clusters can be resident.
+// 4 = one cluster per (item, kv head) (decode_rows.cuh; the caller chooses it by the rows' lengths) or an error:
+// where groups have more than 16 heads, pages don't divide a partition or rows are not 16-byte aligned.
 int rl_attn_decode(int dtype, const void* q, int q_stride, const void* kc, const void* vc,
                    const int32_t* bt, int max_blocks, const int32_t* items, float* part_o,
                    float* part_ml, int max_parts, int* counters, void* out, int out_stride, int nitems,

@@ -8,6 +8,7 @@ compiled extension these functions raise.
 from __future__ import annotations
 
 import ctypes
+import math
 import os
 from concurrent.futures import ThreadPoolExecutor
 from ctypes import c_float, c_int, c_longlong, c_uint, c_void_p
@@ -463,7 +464,7 @@ def attn_decode(q: torch.Tensor, q_stride: int, kcache: torch.Tensor, vcache: to
     impl      0: the best kernel that applies (streaming tensor-core for launches with many partitions,
               one-partition tensor-core, CUDA-core); 1: CUDA-core; 2: one-partition tensor-core or error;
               3: streaming tensor-core or error; 4: one cluster per (item, kv head), partial results
-              merged through distributed shared memory (few rows of similar length) or error
+              merged through distributed shared memory (where attn_decode_rows_pays says so) or error
     """
     _need_cuda(q, kcache, out)
     f = _fn(_attn(head_dim), "rl_attn_decode",
@@ -516,19 +517,31 @@ def attn_decode_rows_cluster(nitems: int, num_kv_heads: int, head_dim: int, devi
     return _rows_cluster[key]
 
 
+# What a decode launch takes in us, by head size, fitted to 2,165 launches on a B200 (kv heads 1, 2, 4 and 8, groups of 4
+# heads, 1 to 128 sequences of 256 to 131,072 keys and up to 800 MB of them: equal lengths, lengths spread over L / 8 to L,
+# one of L beside others of L / 16).
+#   rows: start, per 32-key sub-block of a warp's run at head size 64, bytes per us that one SM takes, bytes per us in all
+#   stream: start, bytes per us, per 128 keys of a warp's run at head size 64, per piece of the longest row to be merged
+#   few: (launches that are too small to stream) start, bytes per us, per partition of the longest row
+_DECODE_FIT = {
+    64: {"rows": (3.5, 0.82, 81e3, 6.3e6), "stream": (8.5, 6.0e6, 0.3, 0.07), "few": (4.9, 4.1e6, 0.044)},
+    128: {"rows": (4.4, 0.52, 72e3, 6.1e6), "stream": (11.0, 5.6e6, 0.8, 0.13), "few": (6.1, 3.5e6, 0.082)},
+}
+_STREAM_MIN_UNITS, _MERGE_MAX_PARTS = 1024, 256        # (kStreamMinUnits, kMaxMergeParts: what launch_decode goes by)
+
+
 def attn_decode_rows_pays(nitems: int, num_kv_heads: int, head_dim: int, max_ctx: int, sum_ctx: int, window: int,
                           device: torch.device) -> bool:
     """Whether the decode kernel of one cluster per (item, kv head) (impl 4) is expected to beat the others for
-    a launch of ``nitems`` rows of at most ``max_ctx`` and together ``sum_ctx`` keys.  Its time goes with the
-    longest row (a row has its cluster's SMs only) times the rows a cluster takes in turn, the streaming
-    kernel's with all keys plus the count and merge of its pieces.  The constants are fitted to times on a
-    B200 (8 kv heads, head sizes 64 and 128, batches of 1 to 64 with 512 to 4,000 keys: equal lengths, lengths spread
-    over L / 8 to L, and one long row among short ones): 3.5 us plus 0.7 us (head size 64) per 32-key sub-block of a
-    warp's run, but no less than the keys' bytes at 6.2 TB/s, plus 0.8 us (less below 1,024 keys) for every mean
-    length that the longest row has beyond one; against 8 us plus the keys' bytes at 3 TB/s.  Over 108 such launches the
-    choice is off by 27 us in all at head size 64 and by 15 us at 128 (constants fitted to equal lengths at head size 64 alone, 4.4 + 1.7 and 8 + bytes
-    at 5.3 TB/s: 68 and 575 us).  21 sequences of 115 to 925 keys: 9.5 us against 13.6; eight of 4,000 at head size 128:
-    25 against 36."""
+    a launch of ``nitems`` rows of at most ``max_ctx`` and together ``sum_ctx`` keys (_DECODE_FIT).  A row has its
+    cluster's SMs only: the time goes with the longest row's run per warp, with the keys that the busiest SM reads, and is
+    no less than all bytes take.  The streaming kernel shares all keys among all warps, and then counts and merges the
+    pieces that it cut the rows into.  A last term keeps launches with one row far longer than the rest away from
+    clusters (their rows are the ones that the fit knows least).
+    Over the fitted launches the choice is 0.5 % longer than the better kernel (before: 4.2 % at head size 64 and 1.7 %
+    at 128, and up to 2.3 times as long above 4,096 keys, which that fit had not seen).  In us, streaming / clusters at head
+    size 64 with 8 kv heads: 21 sequences of 115 to 925 keys 13.6 / 9.5; 1 of 16,384 23 / 11; 8 of 65,536 184 / 153; 128 of
+    1,024 to 8,192 201 / 235; one of 16,384 beside 15 of 1,024 23 / 52, beside 127 of 1,024 67 / 391."""
     csize, resident = attn_decode_rows_cluster(nitems, num_kv_heads, head_dim, device)
     if csize <= 0 or resident <= 0 or max_ctx <= 0:
         return False
@@ -536,20 +549,36 @@ def attn_decode_rows_pays(nitems: int, num_kv_heads: int, head_dim: int, max_ctx
         max_ctx, sum_ctx = min(max_ctx, window), min(sum_ctx, nitems * window)
     if head_dim not in _rows_warps:
         _rows_warps[head_dim] = int(_fn(_attn(head_dim), "rl_attn_decode_rows_warps", [])())
-    warps = _rows_warps[head_dim]
+    return decode_rows_estimate(nitems, num_kv_heads, head_dim, max_ctx, sum_ctx, csize, resident, _rows_warps[head_dim],
+                                sm_count(device)) < 0.0
+
+
+def decode_rows_estimate(nitems: int, num_kv_heads: int, head_dim: int, max_ctx: int, sum_ctx: int, csize: int,
+                         resident: int, warps: int, sms: int) -> float:
+    """Estimated us by which the kernel of a cluster of ``csize`` CTAs of ``warps`` warps per row (``resident`` clusters
+    at once) takes longer than the kernel that runs otherwise."""
+    fit, wide = _DECODE_FIT[head_dim], head_dim / 64.0
     rows = nitems * num_kv_heads
+    mean = max(sum_ctx, 1) / nitems
+    nbytes = sum_ctx * num_kv_heads * head_dim * 4
     groups = 1                      # (as the launcher chooses them)
     if rows > resident:
         groups = next((d for d in range(2, warps) if warps % d == 0 and resident * d >= rows), warps)
-    turns = (rows + resident * groups - 1) // (resident * groups)
-    sub_blocks = (max_ctx + 31) // 32
+    turns = -(-rows // (resident * groups))
     per_row = csize * (warps // groups)
-    nbytes = sum_ctx * num_kv_heads * head_dim * 4
-    run = turns * ((sub_blocks + per_row - 1) // per_row) * (head_dim / 64.0)
-    t_rows = 3.5 + max(0.7 * run, nbytes / 6.2e6)
-    t_rows += 0.8 * (max_ctx * nitems / max(sum_ctx, 1) - 1.0) * min(1.0, max_ctx / 1024.0)
-    t_stream = 8.0 + nbytes / 3.0e6
-    return t_rows < t_stream
+    run = math.ceil((max_ctx + 31) // 32 / per_row)
+    run += (turns - 1) * math.ceil(math.ceil(mean / 32) / per_row)
+    start, per_run, sm_rate, rate = fit["rows"]
+    sm_bytes = (max_ctx + (groups * turns - 1) * mean) / csize * head_dim * 4
+    t_rows = start + max(per_run * wide * run, sm_bytes / sm_rate, nbytes / rate)
+    t_rows += 0.5 * (max_ctx / mean - 1.0) * min(1.0, max_ctx / 4096.0) ** 2
+    parts = (max_ctx + DECODE_PARTITION - 1) // DECODE_PARTITION
+    if rows * parts < _STREAM_MIN_UNITS and parts <= _MERGE_MAX_PARTS:
+        start, rate, per_part = fit["few"]
+        return t_rows - (start + nbytes / rate + per_part * parts)
+    start, rate, per_unit, per_piece = fit["stream"]
+    runs = max(1, math.ceil(sum_ctx * num_kv_heads / DECODE_PARTITION / (sms * warps)))
+    return t_rows - (start + max(nbytes / rate, per_unit * wide * runs) + per_piece * math.ceil(parts / runs))
 
 
 def attn_decode_rope_ok(qkv: torch.Tensor, q_stride: int, kcache: torch.Tensor, vcache: torch.Tensor,
