@@ -536,9 +536,9 @@ def attn_decode_rows_pays(nitems: int, num_kv_heads: int, head_dim: int, max_ctx
     a launch of ``nitems`` rows of at most ``max_ctx`` and together ``sum_ctx`` keys (_DECODE_FIT).  A row has its
     cluster's SMs only: the time goes with the longest row's run per warp, with the keys that the busiest SM reads, and is
     no less than all bytes take.  The streaming kernel shares all keys among all warps, and then counts and merges the
-    pieces that it cut the rows into.  A last term keeps launches with one row far longer than the rest away from
-    clusters (their rows are the ones that the fit knows least).
-    Over the fitted launches the choice is 0.5 % longer than the better kernel (before: 4.2 % at head size 64 and 1.7 %
+    pieces that it cut the rows into.  A last term keeps launches whose longest row has many times the mean length away
+    from clusters: a few us where the two are close, and what clusters lose there they lose by multiples.
+    Over the fitted launches the choice is 0.7 % longer than the better kernel (before: 4.2 % at head size 64 and 1.7 %
     at 128, and up to 2.3 times as long above 4,096 keys, which that fit had not seen).  In us, streaming / clusters at head
     size 64 with 8 kv heads: 21 sequences of 115 to 925 keys 13.6 / 9.5; 1 of 16,384 23 / 11; 8 of 65,536 184 / 153; 128 of
     1,024 to 8,192 201 / 235; one of 16,384 beside 15 of 1,024 23 / 52, beside 127 of 1,024 67 / 391."""
@@ -571,7 +571,7 @@ def decode_rows_estimate(nitems: int, num_kv_heads: int, head_dim: int, max_ctx:
     start, per_run, sm_rate, rate = fit["rows"]
     sm_bytes = (max_ctx + (groups * turns - 1) * mean) / csize * head_dim * 4
     t_rows = start + max(per_run * wide * run, sm_bytes / sm_rate, nbytes / rate)
-    t_rows += 0.5 * (max_ctx / mean - 1.0) * min(1.0, max_ctx / 4096.0) ** 2
+    t_rows += 1.5 * min(max(max_ctx / mean - 4.0, 0.0), 3.0) * min(1.0, max_ctx / 2048.0) ** 2
     parts = (max_ctx + DECODE_PARTITION - 1) // DECODE_PARTITION
     if rows * parts < _STREAM_MIN_UNITS and parts <= _MERGE_MAX_PARTS:
         start, rate, per_part = fit["few"]
