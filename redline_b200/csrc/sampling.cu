@@ -1,4 +1,5 @@
-// Token sampling on the GPU: one CTA per row of float logits.
+// Token sampling on the GPU: one CTA per row of float logits, or a cluster of eight where rows are drawn from a
+// large vocabulary (sample_clusters).
 //
 //   temperature <= 0   greedy: the arg max, the smaller index on ties
 //   temperature  > 0   temperature, then top-k (ties at the k-th value kept), then
@@ -331,11 +332,26 @@ sample_kernel(const float* __restrict__ logits, int vocab, int ld, const float* 
 // read 513 KB for each of them from L2 took 344 us for rows of 128,256 logits (B200, 1 to 32 rows with top-p), this
 // one 47 us at 21 rows together with the wait for the kernel before it.  Every pass here runs over 64 KB in shared memory, and the CTAs' counts or masses meet through distributed shared memory.
 // All selections are over integers (counts, fixed-point mass) or maxima, so they are the same bits in any order: the
-// tokens are those of sample_kernel.  A greedy row costs its first CTA what it did before.
+// tokens are those of sample_kernel.  Of a greedy row's cluster one warp works.
 constexpr int kRowCtas = 8, kRowThreads = 512;
-// Rows from here on: below, a pass of one CTA is as short as a meeting of eight.
-constexpr int kRowVocab = 8192;
 constexpr int kRowMaxBytes = 200 * 1024;
+
+int row_share_bytes(int vocab) { return (((vocab + kRowCtas - 1) / kRowCtas + 3) & ~3) * 4; }
+
+// Whether a launch gets clusters.  draws: 0 no row is drawn (all temperatures are 0), 1 rows are drawn from the whole
+// vocabulary, 2 with top-k or top-p.  Clusters are eight times the CTAs, so few rows and long ones gain; us for one CTA
+// per row / clusters, B200:
+//               vocabulary 8,192                      16,384                       32,000               128,256
+//   top-p       21 rows 184 / 65, 96 237 / 193,       64 355 / 167, 192 556 / 476, 256 965 / 880,       256 3,582 / 2,485,
+//               192 348 / 376, 512 695 / 946          256 568 / 629                512 1,878 / 1,681    512 7,067 / 4,779
+//   no filter   16 rows 16 / 15, 32 19 / 19,          32 27 / 21, 48 30 / 32,      64 51 / 46,          384 584 / 539,
+//               64 32 / 34, 256 65 / 122              128 58 / 70                  96 56 / 66           512 763 / 714
+//   greedy      8 rows 5.5 / 6.5, 256 48 / 53         8 5.5 / 6.5, 256 49 / 54     64 16.3 / 17.0       64 20.9 / 21.8
+// Below 8,192 entries a pass of one CTA is short (4,096: 21 rows with top-p 126 us).
+bool sample_clusters(int rows, int vocab, int draws) {
+  if (draws <= 0 || vocab < 8192 || row_share_bytes(vocab) > kRowMaxBytes) return false;
+  return rows <= vocab / (draws == 1 ? 340 : 80);
+}
 
 struct RowSmem {
   float fscratch[32];
@@ -595,12 +611,16 @@ extern "C" {
 
 int rl_sample_chunks() { return kSampleChunks; }
 
+// Whether rl_sample with these arguments launches clusters (see sample_clusters).
+int rl_sample_clusters(int rows, int vocab, int draws) { return sample_clusters(rows, vocab, draws) ? 1 : 0; }
+
 // scratch: optional [rows * rl_sample_chunks() * 4] floats.  With it, rows whose temperature is <= 0
 // are served by a two-stage arg max that uses the whole GPU instead of one CTA per row.
+// draws: what the rows ask for (see sample_clusters); it decides which kernel runs, not what a row gets.
 int rl_sample(const float* logits, int rows, int vocab, int ld, const float* temperature,
               const int32_t* top_k, const float* top_p, const uint32_t* seed_lo,
               const uint32_t* seed_hi, const int32_t* position, unsigned stream_id,
-              int32_t* out_token, float* out_logprob, float* scratch, cudaStream_t stream) {
+              int32_t* out_token, float* out_logprob, float* scratch, int draws, cudaStream_t stream) {
   if (rows <= 0) return 0;
   ChunkStat* stats = reinterpret_cast<ChunkStat*>(scratch);
   if (stats != nullptr) {
@@ -613,8 +633,7 @@ int rl_sample(const float* logits, int rows, int vocab, int ld, const float* tem
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return static_cast<int>(e);
   }
-  const int share = (((vocab + kRowCtas - 1) / kRowCtas + 3) & ~3) * 4;
-  if (vocab >= kRowVocab && share <= kRowMaxBytes) {
+  if (sample_clusters(rows, vocab, draws)) {
     static std::atomic<bool> raised[64];              // per device
     int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);
@@ -627,7 +646,7 @@ int rl_sample(const float* logits, int rows, int vocab, int ld, const float* tem
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(rows * kRowCtas);
     cfg.blockDim = dim3(kRowThreads);
-    cfg.dynamicSmemBytes = share;
+    cfg.dynamicSmemBytes = row_share_bytes(vocab);
     cfg.stream = stream;
     cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeClusterDimension;

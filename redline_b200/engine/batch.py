@@ -30,6 +30,7 @@ import torch
 
 from ..cache import native
 from ..cache.manager import CacheManager, RequestCache
+from ..ops.kernels import DRAWS_FILTERED, DRAWS_NONE, DRAWS_PLAIN
 
 # The work lists of a step are cut for the mixers that read them: sequences that bring more than
 # one token into tiles of ``tile_rows`` query rows, the context of a single token into partitions
@@ -143,6 +144,7 @@ class StepContext:
     status: torch.Tensor
     has_src: bool = False
     any_sampling: bool = False
+    draws: int = 0           # what the wanted rows ask of the sampler (kernels.DRAWS_NONE, _PLAIN or _FILTERED)
     # the single-token sequences' context lengths (new token included): the longest and their sum
     decode_max_ctx: int = 0
     decode_sum_ctx: int = 0
@@ -254,6 +256,7 @@ class BatchBuilder:
         t = 0
         to = 0
         dec_max = dec_sum = 0
+        draws = DRAWS_NONE
         for s in segments:
             n = len(s.tokens)
             if n == 1:
@@ -262,6 +265,8 @@ class BatchBuilder:
             sp = s.sampling
             fed = s.src_row >= 0
             if sp is not None:
+                if sp.temperature > 0.0 and len(s.want):
+                    draws = max(draws, DRAWS_FILTERED if sp.top_k > 0 or sp.top_p < 1.0 else DRAWS_PLAIN)
                 rows.append((s.cache.rid, s.start_pos, n, s.src_row, to, len(want_flat), len(s.want), 1,
                              sp.temperature, sp.top_p, sp.top_k, sp.seed & 0xFFFFFFFF, (sp.seed >> 32) & 0xFFFFFFFF))
             else:
@@ -327,5 +332,5 @@ class BatchBuilder:
         views = self._views(lay, dev, T, S, R, L)
         return StepContext(T=T, S=S, R=R, num_decode=nd, num_tiles=li, decode_parts=decode_parts,
                            max_items=self.max_seqs, parts_capacity=self.parts_capacity, status=self.status,
-                           has_src=has_src, any_sampling=any_sampling, decode_max_ctx=dec_max,
+                           has_src=has_src, any_sampling=any_sampling, draws=draws, decode_max_ctx=dec_max,
                            decode_sum_ctx=dec_sum, host=hb, **views)

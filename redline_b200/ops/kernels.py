@@ -1617,25 +1617,33 @@ def moe_combine(y: torch.Tensor, weight: torch.Tensor, shared: Optional[torch.Te
 # -------------------------------------------------------------------- sampling
 
 SAMPLE_CHUNKS = 64
+DRAWS_NONE, DRAWS_PLAIN, DRAWS_FILTERED = 0, 1, 2
 
 
 def sample(logits: torch.Tensor, rows: int, temperature: torch.Tensor, top_k: torch.Tensor,
            top_p: torch.Tensor, seed_lo: torch.Tensor, seed_hi: torch.Tensor, position: torch.Tensor,
            out_token: torch.Tensor, out_logprob: Optional[torch.Tensor], stream_id: int = 0,
-           scratch: Optional[torch.Tensor] = None) -> None:
+           scratch: Optional[torch.Tensor] = None, draws: int = DRAWS_FILTERED) -> None:
     """One token per row of float32 logits.  ``scratch`` (float32, rows * SAMPLE_CHUNKS * 4) lets greedy
-    rows use a two-stage arg max over the whole GPU."""
+    rows use a two-stage arg max over the whole GPU.  ``draws``: what the rows ask for as far as the caller knows
+    (DRAWS_NONE: every temperature is 0, DRAWS_PLAIN: no top-k or top-p, DRAWS_FILTERED); it decides which kernel runs
+    (``sample_clusters``), not what a row gets."""
     _need_cuda(logits, out_token)
     if logits.dtype != torch.float32:
         raise KernelError("sample: logits must be float32")
     f = _fn(_lib("sampling", "sampling.cu"), "rl_sample",
             [c_void_p, c_int, c_int, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p,
-             c_uint, c_void_p, c_void_p, c_void_p, c_void_p])
+             c_uint, c_void_p, c_void_p, c_void_p, c_int, c_void_p])
     if scratch is not None and scratch.numel() < rows * SAMPLE_CHUNKS * 4:
         raise KernelError("sample: scratch too small")
     _check(f(_ptr(logits), rows, logits.shape[1], logits.stride(0), _ptr(temperature), _ptr(top_k),
              _ptr(top_p), _ptr(seed_lo), _ptr(seed_hi), _ptr(position), stream_id, _ptr(out_token),
-             _ptr(out_logprob), _ptr(scratch), _stream()), "sample", 2 if scratch is not None else 1)
+             _ptr(out_logprob), _ptr(scratch), draws, _stream()), "sample", 2 if scratch is not None else 1)
+
+
+def sample_clusters(rows: int, vocab: int, draws: int) -> bool:
+    """Whether ``sample`` gives every row of such a launch a cluster of CTAs."""
+    return bool(_fn(_lib("sampling", "sampling.cu"), "rl_sample_clusters", [c_int, c_int, c_int])(rows, vocab, draws))
 
 
 def gather_logprob(logits: torch.Tensor, rows: int, target: torch.Tensor, out: torch.Tensor) -> None:

@@ -17,4 +17,4 @@ class Sampler:
     def sample(self, logits: torch.Tensor, ctx) -> None:
         """Fills tokens[:R] and logprobs[:R] from logits[:R] with the rows' parameters in ctx."""
         kernels.sample(logits, ctx.R, ctx.temperature, ctx.top_k, ctx.top_p, ctx.seed_lo, ctx.seed_hi,
-                       ctx.sample_pos, self.tokens, self.logprobs, scratch=self.scratch)
+                       ctx.sample_pos, self.tokens, self.logprobs, scratch=self.scratch, draws=ctx.draws)

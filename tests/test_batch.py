@@ -51,6 +51,21 @@ def test_mixed_batch_layout():
     assert ctx.host.q_start == [0, 40, 41] and ctx.host.q_len == [40, 1, 3]
 
 
+def test_what_the_wanted_rows_ask_of_the_sampler():
+    """Greedy rows, rows drawn from the whole vocabulary, rows drawn with a filter; parameters of a segment that wants
+    no logits don't count."""
+    cache, b = setup()
+    x, y = cache.open("x"), cache.open("y")
+    cache.reserve(x, 8), cache.reserve(y, 8)
+    for sx, want, draws in ((None, (0,), 0), (RowSampling(0.0, 5, 0.5, 1), (0,), 0), (RowSampling(0.7, 0, 1.0, 1), (0,), 1),
+                            (RowSampling(0.7, 3, 1.0, 1), (0,), 2), (RowSampling(0.7, 0, 0.9, 1), (0,), 2),
+                            (RowSampling(0.7, 0, 0.9, 1), (), 0)):
+        ctx = b.build([Segment(x, [1], 0, want=want, sampling=sx), Segment(y, [2], 0, want=(0,), sampling=RowSampling())])
+        assert ctx.draws == draws
+    assert b.build([Segment(x, [1], 0, want=(0,), sampling=RowSampling(0.7, 0, 0.9, 1)),
+                    Segment(y, [2], 0, want=(0,), sampling=RowSampling(0.7, 0, 1.0, 1))]).draws == 2
+
+
 def test_padding_of_a_decode_batch_and_device_fed_tokens():
     cache, b = setup()
     x, y = cache.open("x"), cache.open("y")

@@ -148,6 +148,23 @@ def test_score_in_portions(models):
     assert eng.runner.cache.num_open() == 0
 
 
+def test_greedy_and_drawn_steps_of_a_large_vocabulary_in_graphs(tmp_path):
+    """Steps whose rows are all greedy, drawn, and drawn with a filter, in one engine with graphs: the tokens of an engine
+    without, and a graph of its own for the steps that draw by clusters."""
+    from redline_b200.runtime import Engine
+    cfg = dict(C.TINY_A, vocab_size=9000)
+    d, w = make_model(tmp_path, cfg, seed=48, sharpen=5.0)
+    prompts = [random_tokens(9000, n, 70 + n) for n in (5, 17, 33)]
+    got = []
+    for graphs in (False, True):
+        eng = Engine(d, dtype="float32", max_seqs=4, max_batched_tokens=64, max_seq_len=128, kv_cache_tokens=512, cuda_graphs=graphs)
+        got.append([[o["output_ids"] for o in eng.generate(prompts, max_new_tokens=6, ignore_eos=True, **kw)]
+                    for kw in (dict(), dict(temperature=0.9, seed=3), dict(temperature=0.9, top_p=0.8, seed=3), dict())])
+        keys = eng._engine.runner._graphs
+    assert got[0] == got[1] and got[0][0] == got[0][3]
+    assert {k[0] for k in keys if k[-1] == "clusters"} == {k[0] for k in keys if k[-1] != "clusters"} == {4}
+
+
 @pytest.mark.parametrize("heads,head_dim", [(32, 64), (17, 128)])
 def test_more_heads_to_a_kv_head_than_clusters_take(heads, head_dim, tmp_path):
     """Groups of more than 16 heads, which the decode kernel of a cluster per row refuses: the layer runs another one."""

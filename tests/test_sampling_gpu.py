@@ -122,6 +122,31 @@ def test_draw_over_a_cluster_equals_the_plain_restatement(V, ld, T, k, p):
     assert np.abs(lp - want.numpy()).max() < 1e-4
 
 
+@pytest.mark.parametrize("V", [8192, 20001, 128256])
+def test_the_kernels_draw_the_same(V):
+    """What the caller says about the rows decides which kernel runs, at row counts on both sides of the lines; the draws
+    are the same, also where what it says is wrong."""
+    R = 70
+    l = torch.randn(R, V, device=DEV) * 3
+    i32 = lambda v: torch.full((R,), v, dtype=torch.int32, device=DEV)      # noqa: E731
+    temp = torch.full((R,), 0.8, device=DEV)
+    temp[::3] = 0.0
+    seed, pos = torch.arange(R, dtype=torch.int32, device=DEV), i32(9)
+    scratch = torch.empty(R * kernels.SAMPLE_CHUNKS * 4, device=DEV)
+    assert not kernels.sample_clusters(1, V, kernels.DRAWS_NONE) and kernels.sample_clusters(70, V, kernels.DRAWS_FILTERED)
+    assert kernels.sample_clusters(70, V, kernels.DRAWS_PLAIN) == (V == 128256)
+    assert not kernels.sample_clusters(1, 8191, kernels.DRAWS_FILTERED)
+    for k, p in ((0, 1.0), (40, 0.9)):
+        got = []
+        for draws in (kernels.DRAWS_NONE, kernels.DRAWS_PLAIN, kernels.DRAWS_FILTERED):
+            tok, lp = i32(-1), torch.empty(R, device=DEV)
+            kernels.sample(l, R, temp, i32(k), torch.full((R,), p, device=DEV), seed, i32(0), pos, tok, lp, scratch=scratch,
+                           draws=draws)
+            got.append((tok, lp))
+        assert all(torch.equal(t, got[0][0]) and (x - got[0][1]).abs().max() < 1e-4 for t, x in got)
+        assert torch.equal(got[0][0][::3], l.argmax(-1).int()[::3])
+
+
 @pytest.mark.parametrize("T,k,p", [(1.0, 0, 0.95), (1.4, 200, 0.9), (3.0, 40000, 0.8)])
 def test_draw_at_a_served_vocabulary(T, k, p):
     """128,256 logits, 64 KB of a row to a CTA (more than a kernel has without asking): tokens drawn from flat and from
