@@ -30,9 +30,11 @@
 // slots' exponentials, of 3,700 that a pair of tiles takes, the rest their other instructions and the hand-overs.  One
 // thread to a row takes the maximum of every score once (two to a row, each of which has to know the whole row's
 // maximum, took it twice) and needs no exchange between the two at a tile's P (head size 128) and at an item's end.
-// Measured (one sequence, 32 / 8 heads; in brackets two threads to a row): head size 64, 333 tokens 15.2 us (17.4),
-// 2,048 44.5 (48.5), 4,096 135.5 (141.5), 8,192 482 (484), 16,384 1,778 (1,760); head size 128, 333 tokens 21.8 (26.4),
-// 2,048 70.6 (79.6), 8,192 837 (917), 16,384 3,149 (3,453).
+// Measured (one sequence, 32 / 8 heads; in brackets two threads to a row): head size 64, 333 tokens 15.2 us (17.3),
+// 2,048 44.5 (48.3), 8,192 475 (482), 16,384 1,779 (1,752), 2,048 behind 6,144 keys 225 (222), behind 12,288 406 (398);
+// head size 128, 333 tokens 21.9 (26.4), 2,048 70.4 (79.5), 8,192 834 (918), 16,384 3,146 (3,464), 2,048 behind 12,288
+// 724 (795).  So long rows at head size 64 are 1 to 2 % slower: half the row warps hide less of the hand-overs.
+// The two give the same bits: a row's denominator is summed in the two threads' chains still.
 // Warp roles: warps 0-3 rows of slot 0, warps 4-7 rows of slot 1 (warp w owns TMEM lanes
 // 32 (w % 4) ..), warp 8 brings both Q tiles once per item and the K tiles, warp 9 the V tiles,
 // from the paged cache with 16-byte cp.async copies (zero-filled outside the live keys), lane 0
@@ -516,7 +518,9 @@ prefill_attn_tc_kernel(const PrefillArgs<bf16> a, int tiles, int* status) {
       const int pos_r = pos0 + r;
       const int win_r = (a.window > 0 && pos_r + 1 > a.window) ? pos_r + 1 - a.window : 0;
       const int lim_r = r < rows ? pos_r : -1;             // the row's live keys are win_r .. lim_r (none for a row past the tile's rows)
-      float m_ref = -INFINITY, l = 0.f;                   // the maximum that P is scaled by (log2 units), the denominator
+      // the maximum that P is scaled by (log2 units), the denominator's parts of the first and the second 64 keys of
+      // every tile (two chains of half the length; added at the item's end)
+      float m_ref = -INFINITY, l[2] = {0.f, 0.f};
       for (int i = 0; i < w.nt && ok; ++i) {
         const int n = g_base + i;
         const int t0 = w.k_begin + i * kTcKeys;
@@ -565,13 +569,20 @@ prefill_attn_tc_kernel(const PrefillArgs<bf16> a, int tiles, int* status) {
           m_ref = m_new;
         } else if (__any_sync(0xffffffffu, m_new > m_ref + kTcGrow)) {
           alpha = m_new == m_ref ? 1.f : ex2_approx(m_ref - m_new);                       // 2^(-inf) = 0
-          l *= alpha;
+          l[0] *= alpha;
+          l[1] *= alpha;
           m_ref = m_new;
           moved = true;
         }
         const float m_use = m_ref == -INFINITY ? 0.f : m_ref;  // a row without a live key so far
         const uint64_t sc2 = f32x2(sc, sc), nm2 = f32x2(-m_use, -m_use);
         uint64_t sum_a = f32x2(0.f, 0.f), sum_b = sum_a;
+        auto add_sums = [](float& part, uint64_t a2, uint64_t b2) {
+          float s0, s1, s2, s3;
+          f32x2_split(a2, s0, s1);
+          f32x2_split(b2, s2, s3);
+          part += (s0 + s1) + (s2 + s3);
+        };
         // 32 scores become 16 columns of P (two keys to a column)
         auto exponentials = [&](uint32_t* v) {
 #pragma unroll
@@ -618,22 +629,20 @@ prefill_attn_tc_kernel(const PrefillArgs<bf16> a, int tiles, int* status) {
           if (lane == 0) mbar_arrive(&sh->s_free[s]);
         }
         tmem_st16(p_addr + 16, vb);
+        const uint64_t first_a = sum_a, first_b = sum_b;
+        sum_a = sum_b = f32x2(0.f, 0.f);
         mask(vc, 2);
         exponentials(vc);
         tmem_st16(p_addr + 32, vc);
         mask(va, 3);
         exponentials(va);
         tmem_st16(p_addr + 48, va);
-        {
-          float s0, s1, s2, s3;
-          f32x2_split(sum_a, s0, s1);
-          f32x2_split(sum_b, s2, s3);
-          l += (s0 + s1) + (s2 + s3);
-        }
         tmem_wait_st();
         tc_fence_before();
         __syncwarp();
         if (lane == 0) mbar_arrive(&sh->p_ready[s]);
+        add_sums(l[0], first_a, first_b);                  // (behind the hand-over: the product starts meanwhile)
+        add_sums(l[1], sum_a, sum_b);
       }
       if (!ok) break;
       // ---- the item's rows: O / denominator, once its last product is done
@@ -641,7 +650,8 @@ prefill_attn_tc_kernel(const PrefillArgs<bf16> a, int tiles, int* status) {
       ok = __all_sync(0xffffffffu, ok);
       if (!ok) break;
       tc_fence_after();
-      const float inv = l > 0.f ? 1.f / l : 0.f;
+      const float l_all = l[0] + l[1];
+      const float inv = l_all > 0.f ? 1.f / l_all : 0.f;
       bf16* dst = a.out + static_cast<size_t>(w.tok0 + (r < rows ? r : 0)) * a.out_stride + (w.head0 + s) * kD;
 #pragma unroll
       for (int c0 = 0; c0 < kD; c0 += 32) {
