@@ -342,20 +342,24 @@ int rl_embedding(const int32_t* ids, const void* table, int table_dtype, float* 
 }
 
 // act_dtype: type of `delta` and `out`; w_dtype: type of `weight`.
-int rl_add_rmsnorm(float* residual, const void* delta, const void* weight, int w_dtype, void* out,
+// (delta: of out's type or float)
+int rl_add_rmsnorm(float* residual, const void* delta, int d_dtype, const void* weight, int w_dtype, void* out,
                    int act_dtype, const int32_t* rows_idx, int rows, int hidden, float eps,
                    cudaStream_t stream) {
   if (rows <= 0) return 0;
   // eight columns per thread where the row allows it (then, up to 4,096 columns, the row stays in registers)
   const int th = hidden % 8 == 0 ? row_threads(hidden / 8) : row_threads(hidden);
-#define RL_NORM_CASE(TA, TW)                                                                 \
-  launch_kernel(add_rmsnorm_kernel<TA, TA, TW>, dim3(rows), dim3(th), 0, stream,                                    \
-      residual, static_cast<const TA*>(delta), static_cast<const TW*>(weight),               \
+#define RL_NORM_CASE(TA, TD, TW)                                                             \
+  launch_kernel(add_rmsnorm_kernel<TA, TD, TW>, dim3(rows), dim3(th), 0, stream,                                    \
+      residual, static_cast<const TD*>(delta), static_cast<const TW*>(weight),               \
       static_cast<TA*>(out), rows_idx, hidden, eps)
-  if (act_dtype == RL_F32 && w_dtype == RL_F32) RL_NORM_CASE(float, float);
-  else if (act_dtype == RL_F32) RL_NORM_CASE(float, bf16);
-  else if (w_dtype == RL_F32) RL_NORM_CASE(bf16, float);
-  else RL_NORM_CASE(bf16, bf16);
+  if (act_dtype == RL_F32 && d_dtype != RL_F32) return static_cast<int>(cudaErrorInvalidValue);
+  if (act_dtype == RL_F32 && w_dtype == RL_F32) RL_NORM_CASE(float, float, float);
+  else if (act_dtype == RL_F32) RL_NORM_CASE(float, float, bf16);
+  else if (d_dtype == RL_F32 && w_dtype == RL_F32) RL_NORM_CASE(bf16, float, float);
+  else if (d_dtype == RL_F32) RL_NORM_CASE(bf16, float, bf16);
+  else if (w_dtype == RL_F32) RL_NORM_CASE(bf16, bf16, float);
+  else RL_NORM_CASE(bf16, bf16, bf16);
 #undef RL_NORM_CASE
   RL_LAUNCH_END();
 }

@@ -148,9 +148,10 @@ class StepContext:
     # the single-token sequences' context lengths (new token included): the longest and their sum
     decode_max_ctx: int = 0
     decode_sum_ctx: int = 0
-    # every sublayer that adds its output product to the stream as a float32 sum in a step of 64 rows does so at any
-    # number of rows (set for scoring; other prompt steps round that product to the activation type before the add)
+    # output products of sublayers stay float32 until they are added to the stream, where the part and the norm that adds
+    # them can (set for scoring; other prompt steps of more than 64 rows round them to the activation type first)
     float32_sums: bool = False
+    out_float32: bool = False                  # set and cleared by the block: the running part may leave float32
     host: Optional["HostBatch"] = None
     profiler: Optional[object] = None          # engine.profiler.OpProfiler while per-op profiling is on
     # a norm handed over between parts (parts.base.NormHandover); set and cleared by the block
@@ -158,6 +159,7 @@ class StepContext:
     hand_in: Optional[object] = None           # what the part before left for the running part's norm
     hand_out: Optional[object] = None          # what the running part leaves
     block_next_norm: Optional[object] = None   # set by the model: the first norm of the block after this one
+    block_after_norm: Optional[object] = None  # set by the model: the norm that adds what this block leaves pending
     block_next: Optional[object] = None        # set by the model: the block after this one (None after the last)
     block_stream: Optional[object] = None      # set by a block whose sublayers read the stream itself: its float32 rows
     block_hand: Optional[object] = None        # carried from a block's last part to the next block

@@ -188,12 +188,13 @@ class DecoderModel:
             # (the block after this one may take over its first norm from this block's last kernel)
             ctx.block_next = self.blocks[order[i + 1].layer] if i + 1 < len(order) else None
             ctx.block_next_norm = ctx.block_next.first_norm() if ctx.block_next is not None else None
+            ctx.block_after_norm = ctx.block_next_norm if ctx.block_next is not None else self.final_norm
             if self.nvtx_layers:
                 torch.cuda.nvtx.range_push(f"layer call {i} (layer {call.layer})")
             pending = self.blocks[call.layer].forward(residual, pending, ctx, caches[i], states[i])
             if self.nvtx_layers:
                 torch.cuda.nvtx.range_pop()
-        ctx.block_hand = ctx.block_next_norm = ctx.block_normed = ctx.block_next = None
+        ctx.block_hand = ctx.block_next_norm = ctx.block_after_norm = ctx.block_normed = ctx.block_next = None
         return residual, pending
 
     def forward(self, ctx, caches, states, logits: torch.Tensor) -> torch.Tensor:

@@ -114,16 +114,16 @@ def embedding(ids: torch.Tensor, table: torch.Tensor, out: torch.Tensor, status:
 def add_rmsnorm(residual: torch.Tensor, delta: Optional[torch.Tensor], weight: torch.Tensor,
                 out: torch.Tensor, eps: float, rows_idx: Optional[torch.Tensor] = None,
                 rows: Optional[int] = None) -> None:
-    """residual += delta (if given); out = rmsnorm(residual) * weight.  With
+    """residual += delta (if given; of out's type or float32); out = rmsnorm(residual) * weight.  With
     ``rows_idx`` only those rows are normalised (out row i <- row rows_idx[i]) and
     residual is left as it is."""
     _need_cuda(residual, weight, out)
     n = rows if rows is not None else (rows_idx.numel() if rows_idx is not None else residual.shape[0])
-    f = _fn(_ew(), "rl_add_rmsnorm", [c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_int, c_void_p,
+    f = _fn(_ew(), "rl_add_rmsnorm", [c_void_p, c_void_p, c_int, c_void_p, c_int, c_void_p, c_int, c_void_p,
                                        c_int, c_int, c_float, c_void_p])
-    if delta is not None and delta.dtype != out.dtype:
-        raise KernelError("add_rmsnorm: delta and out must have the same dtype")
-    _check(f(_ptr(residual), _ptr(delta), _ptr(weight), _code(weight.dtype), _ptr(out), _code(out.dtype),
+    if delta is not None and delta.dtype not in (out.dtype, torch.float32):
+        raise KernelError("add_rmsnorm: delta must have out's dtype or be float32")
+    _check(f(_ptr(residual), _ptr(delta), _code(out.dtype if delta is None else delta.dtype), _ptr(weight), _code(weight.dtype), _ptr(out), _code(out.dtype),
              _ptr(rows_idx), n, residual.shape[-1], float(eps), _stream()), "add_rmsnorm")
 
 
@@ -359,11 +359,6 @@ def mid_rows(rows: int, *weights: torch.Tensor) -> bool:
     aligned rows.  ``REDLINE_MID_PRODUCTS=0`` says no (for comparisons)."""
     if rows <= 0 or rows > MID_ROUTED_ROWS or os.environ.get("REDLINE_MID_PRODUCTS", "1") == "0":
         return False
-    return tc_weights(*weights)
-
-
-def tc_weights(*weights: torch.Tensor) -> bool:
-    """Whether gemm_tc and gemm_mid take products over these weights (with activations in rows of a workspace)."""
     return all(w.dtype == torch.bfloat16 and w.is_contiguous() and w.shape[1] % 8 == 0 and w.data_ptr() % 16 == 0
                for w in weights)
 

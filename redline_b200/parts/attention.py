@@ -102,7 +102,8 @@ class GQAttention(Mixer):
         linear(x, self.w_qkv, qkv)
         op_mark(ctx, "qkv_proj", self.w_qkv, T)
         attn = self._attend(qkv, ctx, cache)
-        out = rt.workspace.get("mixer.out", (rt.max_tokens, p.hidden_size), rt.dtype)[:T]
+        dtype = torch.float32 if ctx.out_float32 and self.b_o is None else rt.dtype
+        out = rt.workspace.get("mixer.out", (rt.max_tokens, p.hidden_size), dtype)[:T]
         linear(attn, self.w_o, out)
         if self.b_o is not None:
             kernels.add_bias(out, self.b_o)
@@ -119,8 +120,6 @@ class GQAttention(Mixer):
             return self._into_skinny(residual, rms, ctx, cache)
         if kernels.mid_rows(T, self.w_qkv, self.w_o):
             return self._into_mid(residual, rms, ctx, cache)
-        if ctx.float32_sums and kernels.tc_weights(self.w_qkv, self.w_o):
-            return self._into_wide(residual, rms, ctx, cache)
         return False
 
     def _into_skinny(self, residual, rms, ctx, cache) -> bool:
@@ -169,22 +168,6 @@ class GQAttention(Mixer):
                          hand_out=None if out is None else (out.norm.rms_params()[0], out.xw, out.sums))
         op_mark(ctx, "o_proj+add", self.w_o, T)
         ctx.hand_out = out
-        return True
-
-    def _into_wide(self, residual, rms, ctx, cache) -> bool:
-        """More rows, in steps that keep float32 sums (``ctx.float32_sums``): the output product adds its
-        accumulators to the stream as they are."""
-        rt = self.rt
-        T = ctx.T
-        xn = rt.workspace.get("block.normed", (rt.max_tokens, residual.shape[1]), rt.dtype)[:T]
-        kernels.add_rmsnorm(residual, None, rms[0], xn, rms[1], rows=T)
-        op_mark(ctx, "rmsnorm", nbytes=T * residual.shape[1] * 6.0)
-        qkv = rt.workspace.get("attn.qkv", (rt.max_tokens, self.qkv_size), rt.dtype)[:T]
-        linear(xn, self.w_qkv, qkv)
-        op_mark(ctx, "qkv_proj", self.w_qkv, T)
-        attn = self._attend(qkv, ctx, cache)
-        kernels.gemm_tc(attn, self.w_o, residual, kernels.EPI_ADD_RESIDUAL)
-        op_mark(ctx, "o_proj+add", self.w_o, T)
         return True
 
     def decode_variant(self, ctx) -> int:

@@ -150,6 +150,8 @@ class Part:
 
 
 class Norm(Part):
+    adds_float32 = False          # whether add_norm takes a float32 delta for an output of another type
+
     def add_norm(self, residual: torch.Tensor, delta: Optional[torch.Tensor], out: torch.Tensor,
                  rows_idx: Optional[torch.Tensor] = None, rows: Optional[int] = None) -> None:
         """residual (float32) += delta; out = norm(residual).  With ``rows_idx`` only

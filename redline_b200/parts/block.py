@@ -33,6 +33,7 @@ class PreNormBlock(Block):
         rt = self.rt
         T = ctx.T
         x = None
+        wide = getattr(ctx, "float32_sums", False)        # (the parts may leave float32 for the norm that adds it)
         hand, ctx.block_hand = ctx.block_hand, None       # from the block before, for this block's first norm
         # small batches: the mixer and the feed-forward may fuse the norm into their first
         # kernel and the residual add into their last (nothing is then left pending)
@@ -48,7 +49,10 @@ class PreNormBlock(Block):
             x = rt.workspace.get("block.normed", (rt.max_tokens, residual.shape[1]), rt.dtype)[:T]
             self.mixer_norm.add_norm(residual, pending, x, rows=T)
             op_mark(ctx, "add+rmsnorm", nbytes=self._norm_bytes(residual, pending, x))
+            if wide:
+                ctx.out_float32 = self._adds_float32(self.ffn_norm if self.ffn is not None else ctx.block_after_norm)
             a = self.mixer.forward(x, ctx, cache, state)
+            ctx.out_float32 = False
         if self.ffn is None:               # a layer with a mixer only: its output is what is left to add
             ctx.block_hand = hand if a is None else None
             return a
@@ -62,7 +66,16 @@ class PreNormBlock(Block):
             x = rt.workspace.get("block.normed", (rt.max_tokens, residual.shape[1]), rt.dtype)[:T]
         self.ffn_norm.add_norm(residual, a, x, rows=T)
         op_mark(ctx, "add+rmsnorm", nbytes=self._norm_bytes(residual, a, x))
-        return self.ffn.forward(x, ctx)
+        if wide:
+            ctx.out_float32 = self._adds_float32(ctx.block_after_norm)
+        f = self.ffn.forward(x, ctx)
+        ctx.out_float32 = False
+        return f
+
+    @staticmethod
+    def _adds_float32(norm) -> bool:
+        """Whether ``norm``, which adds the running part's output to the stream, takes it in float32."""
+        return getattr(norm, "adds_float32", False)
 
     @staticmethod
     def _norm_bytes(residual, delta, out) -> float:

@@ -9,7 +9,7 @@ fuse the norm before and the add behind are SiLU's."""
 from __future__ import annotations
 
 from dataclasses import dataclass
-from typing import Dict
+from typing import Dict, Optional
 
 import torch
 
@@ -78,23 +78,11 @@ class SwiGLUMLP(FeedForward):
                 + self.w_down.numel() * self.w_down.element_size())
 
     def forward(self, x, ctx) -> torch.Tensor:
-        return self.run(x, ctx, "ffn")
+        return self.run(x, ctx, "ffn", torch.float32 if ctx.out_float32 and self.b_down is None else self.rt.dtype)
 
-    def run(self, x, ctx, name: str) -> torch.Tensor:
+    def run(self, x, ctx, name: str, out_dtype: Optional[torch.dtype] = None) -> torch.Tensor:
         """The feed-forward with its buffers named after ``name`` (a part that runs one beside its own
         feed-forward, a shared expert for instance, names another)."""
-        p, rt = self.params, self.rt
-        T = ctx.T
-        act = self._activated(x, ctx, name)
-        out = rt.workspace.get(name + ".out", (rt.max_tokens, p.hidden_size), rt.dtype)[:T]
-        linear(act, self.w_down, out)
-        if self.b_down is not None:
-            kernels.add_bias(out, self.b_down)
-        op_mark(ctx, "down_proj", self.w_down, T)
-        return out
-
-    def _activated(self, x, ctx, name: str) -> torch.Tensor:
-        """act(gate(x)) * up(x)."""
         p, rt = self.params, self.rt
         T = ctx.T
         ws = rt.workspace
@@ -120,7 +108,12 @@ class SwiGLUMLP(FeedForward):
             else:
                 kernels.gated_act(gu, act, kernels.ACTIVATIONS[self.params.activation], bias=self.b_gate_up)
         op_mark(ctx, "gate_up+swiglu" if self.silu else "gate_up+act", self.w_gate_up, T)
-        return act
+        out = ws.get(name + ".out", (rt.max_tokens, p.hidden_size), out_dtype or rt.dtype)[:T]
+        linear(act, self.w_down, out)
+        if self.b_down is not None:
+            kernels.add_bias(out, self.b_down)
+        op_mark(ctx, "down_proj", self.w_down, T)
+        return out
 
     def forward_into(self, residual, norm, ctx) -> bool:
         rt = self.rt
@@ -133,8 +126,6 @@ class SwiGLUMLP(FeedForward):
             return self._into_skinny(residual, rms, ctx)
         if kernels.mid_rows(T, self.w_gate_up, self.w_down):
             return self._into_mid(residual, rms, ctx)
-        if ctx.float32_sums and kernels.tc_weights(self.w_gate_up, self.w_down):
-            return self._into_wide(residual, rms, ctx)
         return False
 
     def _into_skinny(self, residual, rms, ctx) -> bool:
@@ -184,17 +175,4 @@ class SwiGLUMLP(FeedForward):
                          hand_out=None if out is None else (out.norm.rms_params()[0], out.xw, out.sums))
         op_mark(ctx, "down_proj+add", self.w_down, T)
         ctx.hand_out = out
-        return True
-
-    def _into_wide(self, residual, rms, ctx) -> bool:
-        """More rows, in steps that keep float32 sums (``ctx.float32_sums``): the down product adds its accumulators
-        to the stream as they are."""
-        rt = self.rt
-        T = ctx.T
-        xn = rt.workspace.get("block.normed", (rt.max_tokens, residual.shape[1]), rt.dtype)[:T]
-        kernels.add_rmsnorm(residual, None, rms[0], xn, rms[1], rows=T)
-        op_mark(ctx, "rmsnorm", nbytes=T * residual.shape[1] * 6.0)
-        act = self._activated(xn, ctx, "ffn")
-        kernels.gemm_tc(act, self.w_down, residual, kernels.EPI_ADD_RESIDUAL)
-        op_mark(ctx, "down_proj+add", self.w_down, T)
         return True

@@ -28,6 +28,8 @@ class RMSNormParams:
 
 @register("norm", "rmsnorm")
 class RMSNorm(Norm):
+    adds_float32 = True
+
     def tensors(self) -> Dict[str, TensorSpec]:
         return {"weight": TensorSpec((self.params.size,))}
 

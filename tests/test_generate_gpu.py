@@ -203,6 +203,25 @@ def test_score_over_several_blocks(n, batched, rows, own, dtype, models, monkeyp
     assert eng.runner.cache.num_open() == 0
 
 
+def test_score_without_memory_for_more_logits(models, monkeypatch):
+    """The buffer beside the engine's own cannot be had: its own serves, in blocks of as many rows."""
+    from redline_b200.engine.engine import Engine
+    d, _ = models["tiny_a"]
+    opts = dict(dtype="float32", max_num_seqs=2, max_num_batched_tokens=64, max_logit_rows=10, max_seq_len=256, kv_cache_tokens=512)
+    toks = random_tokens(512, 150, 8)
+    want = Engine(d, **opts).score(toks)
+    eng, empty = Engine(d, **opts), torch.empty
+
+    def full(*shape, **kw):
+        if shape == ((64, 512),):
+            raise torch.OutOfMemoryError("no memory")
+        return empty(*shape, **kw)
+
+    monkeypatch.setattr(torch, "empty", full)
+    got = eng.score(toks)
+    assert np.abs(np.array(got) - np.array(want)).max() < 1e-5
+
+
 @pytest.mark.parametrize("design,name,dtype", [("vizotar", "mix", "float32"), ("vizotar", "calm", "bfloat16"),
                                                ("kapitar", "mix", "float32"), ("kapitar", "plain", "bfloat16")])
 def test_score_of_models_with_states_and_streams(design, name, dtype, tmp_path, monkeypatch):
@@ -243,13 +262,13 @@ def test_scored_portions_add_float32_sums(T, tmp_path):
     ctx = run.builder.build([Segment(rc, toks, 0)])
     ctx.float32_sums = True
     residual, pending = run.model.body(ctx, run._caches, run._states)
-    assert pending is None
+    assert pending.dtype == torch.float32
     attn, act = (run.rt.workspace.get(n, (256, x.shape[1]), torch.bfloat16)[:T].double().cpu() for n, x in (
         ("attn.out", w["model.layers.0.self_attn.o_proj.weight"]), ("ffn.act", w["model.layers.0.mlp.down_proj.weight"])))
     o, down = w["model.layers.0.self_attn.o_proj.weight"].double(), w["model.layers.0.mlp.down_proj.weight"].double()
     want = w["model.embed_tokens.weight"].double()[toks] + attn @ o.T + act @ down.T
     bound = 2.0 ** -16 * (attn.abs() @ o.abs().T + act.abs() @ down.abs().T) + 2.0 ** -22 * want.abs()
-    assert ((residual.double().cpu() - want).abs() <= bound).all()
+    assert ((residual.double().cpu() + pending.double().cpu() - want).abs() <= bound).all()
     run.close("s")
 
 

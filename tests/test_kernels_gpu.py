@@ -67,6 +67,23 @@ def test_add_rmsnorm(dtype, hidden, eps):
     close(out, ref, TOL[dtype])
 
 
+@pytest.mark.parametrize("wdtype", ["float32", "bfloat16"])
+@pytest.mark.parametrize("hidden", [200, 203, 2048, 8192])
+def test_add_rmsnorm_adds_a_float32_addend(hidden, wdtype):
+    """A float32 addend of bfloat16 outputs: the stream is the float32 sum of both, bit for bit, also in gathered rows."""
+    res, delta = torch.randn(7, hidden, device=DEV), torch.randn(7, hidden, device=DEV)
+    w = (1 + 0.1 * torch.randn(hidden, device=DEV)).to(DT[wdtype])
+    total = res + delta
+    ref = (total.double() * torch.rsqrt(total.double().pow(2).mean(-1, keepdim=True) + 1e-5) * w.double()).cpu()
+    out, some = (torch.empty(n, hidden, device=DEV, dtype=torch.bfloat16) for n in (7, 2))
+    idx = torch.tensor([5, 0], dtype=torch.int32, device=DEV)
+    kernels.add_rmsnorm(res, delta, w, some, 1e-5, rows_idx=idx)
+    kernels.add_rmsnorm(res, delta, w, out, 1e-5)
+    assert torch.equal(res, total)
+    close(out, ref, TOL["bfloat16"])
+    assert torch.equal(some, out[idx.long()])
+
+
 @pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
 @pytest.mark.parametrize("inter", [704, 328, 1000])
 def test_swiglu(dtype, inter):
