@@ -137,7 +137,9 @@ struct Piece<T, 1> {
 // keys AND values before it multiplies any (16 pieces of each where rows have 128 entries or less in 16 bits; rows of up
 // to 256 in batches of four; of longer rows a piece when it is multiplied: the sums alone take the registers there), and reads the work item and its pages while the kernel before still runs.  Decode steps of eight such
 // sequences, with the merge below: 0.52 -> 0.48 ms (two layers of 64 / 128 entries and two maps), 0.36 -> 0.31 ms (three of
-// 128 / 128 and 96 entries).
+// 128 / 128 and 96 entries).  Where sequences fill the chip the registers that the pieces take (fewer CTAs to an SM) cost less
+// than the loads ahead gain: a launch over 1 / 8 / 64 / 128 sequences of 540 keys, with the merge, 64 / 128 entries and two maps
+// 30 / 42 / 103 / 182 -> 20 / 23 / 89 / 164 us, 128 / 128 and one map 18 / 25 / 64 / 112 -> 10 / 12 / 48 / 89.
 template <typename T>
 __global__ void __launch_bounds__(kThreads)
 maps_decode_kernel(const MapsDecodeArgs<T> a) {

@@ -17,12 +17,12 @@
 // Measured on a B200 (float32; one launch over weights that are not in L2; in brackets the kernel of 64 x 64 tiles, 4 x 4
 // outputs a thread and one chain over all of K that stood here before):
 //   rows   N 3072 K 2048    N 2048 K 2048    N 16384 K 2048   N 2048 K 8192    N 128256 K 2048
-//      1    8.0 us (152)     6.7 us (151)     30 us (232)      22 us (602)      181 us (1181; 5.8 TB/s)
-//      4   12.2   (152)      8.1   (152)      38   (233)       30   (589)       221   (1191)
-//     16   22     (152)     21     (151)      66   (237)       77   (605)       437   (1226)
-//     64   50     (154)     33     (153)     149   (255)      127   (613)
-//    210  141     (303)     75     (210)     505   (690)      280   (626)
-//    512  219     (390)    147     (343)    1020  (1367)      557  (1214; 31 TFLOP/s)
+//      1    8.1 us (152)     7.1 us (152)     31 us (232)      27 us (615)      183 us (1182; 5.7 TB/s)
+//      4   12.1   (153)     10.3   (153)      38   (233)       30   (610)       221   (1191)
+//     16   25     (152)     21     (153)      66   (237)       76   (623)       434   (1227)
+//     64   49     (155)     32     (155)     148   (255)      126   (617)      1013   (1372)
+//    210  117     (288)     74     (243)     479   (690)      280   (587)
+//    512  218     (389)    146     (356)    1015  (1367)      555  (1119; 31 TFLOP/s)
 // Their error against float64 is a third of the one chain's (2.9e-7 against 8e-7 at K = 2048).
 #include <atomic>
 #include <type_traits>

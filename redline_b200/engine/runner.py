@@ -158,7 +158,7 @@ class ModelRunner:
             self.profiler.begin("decode" if single == len(segments) else ("prefill" if single == 0 else "mixed"))
         if bucket or chunk is not None:
             key = (bucket, self.model.decode_variants(ctx)) if bucket else chunk
-            if kernels.sample_clusters(ctx.R, self.vocab_size, ctx.draws):      # (another kernel, another graph)
+            if ctx.draws and kernels.sample_clusters(ctx.R, self.vocab_size, ctx.draws):     # (another kernel, another graph)
                 key += ("clusters",)
             g = self._graphs.get(key)
             if g is None:

@@ -51,13 +51,15 @@ def _fn(lib: ctypes.CDLL, name: str, argtypes):
 # that a launch took, pointers wrapped in c_void_p another 2 (plain integers do as well).  A prompt of 333 tokens
 # went from 3.06 to 1.98 ms with them and the workspace's kept views.
 # (A torch without CUDA has neither function: the module still imports there, and a launch says why it cannot be.)
-_raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)
-_device_index = getattr(torch._C, "_cuda_getDevice", None)
+def _no_cuda(*_):
+    raise KernelError("redline_b200 kernels need a torch that was built with CUDA")
+
+
+_raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", _no_cuda)
+_device_index = getattr(torch._C, "_cuda_getDevice", _no_cuda)
 
 
 def _stream() -> int:
-    if _raw_stream is None or _device_index is None:
-        raise KernelError("redline_b200 kernels need a torch that was built with CUDA")
     return _raw_stream(_device_index())
 
 
@@ -121,9 +123,13 @@ def add_rmsnorm(residual: torch.Tensor, delta: Optional[torch.Tensor], weight: t
     n = rows if rows is not None else (rows_idx.numel() if rows_idx is not None else residual.shape[0])
     f = _fn(_ew(), "rl_add_rmsnorm", [c_void_p, c_void_p, c_int, c_void_p, c_int, c_void_p, c_int, c_void_p,
                                        c_int, c_int, c_float, c_void_p])
-    if delta is not None and delta.dtype not in (out.dtype, torch.float32):
-        raise KernelError("add_rmsnorm: delta must have out's dtype or be float32")
-    _check(f(_ptr(residual), _ptr(delta), _code(out.dtype if delta is None else delta.dtype), _ptr(weight), _code(weight.dtype), _ptr(out), _code(out.dtype),
+    code = _code(out.dtype)
+    d_code = code
+    if delta is not None and delta.dtype != out.dtype:
+        if delta.dtype != torch.float32:
+            raise KernelError("add_rmsnorm: delta must have out's dtype or be float32")
+        d_code = 0
+    _check(f(_ptr(residual), _ptr(delta), d_code, _ptr(weight), _code(weight.dtype), _ptr(out), code,
              _ptr(rows_idx), n, residual.shape[-1], float(eps), _stream()), "add_rmsnorm")
 
 

@@ -52,7 +52,8 @@ class PreNormBlock(Block):
             if wide:
                 ctx.out_float32 = self._adds_float32(self.ffn_norm if self.ffn is not None else ctx.block_after_norm)
             a = self.mixer.forward(x, ctx, cache, state)
-            ctx.out_float32 = False
+            if wide:
+                ctx.out_float32 = False
         if self.ffn is None:               # a layer with a mixer only: its output is what is left to add
             ctx.block_hand = hand if a is None else None
             return a
@@ -66,8 +67,9 @@ class PreNormBlock(Block):
             x = rt.workspace.get("block.normed", (rt.max_tokens, residual.shape[1]), rt.dtype)[:T]
         self.ffn_norm.add_norm(residual, a, x, rows=T)
         op_mark(ctx, "add+rmsnorm", nbytes=self._norm_bytes(residual, a, x))
-        if wide:
-            ctx.out_float32 = self._adds_float32(ctx.block_after_norm)
+        if not wide:
+            return self.ffn.forward(x, ctx)
+        ctx.out_float32 = self._adds_float32(ctx.block_after_norm)
         f = self.ffn.forward(x, ctx)
         ctx.out_float32 = False
         return f
