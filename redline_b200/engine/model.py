@@ -18,6 +18,7 @@ from ..parts.spec import CacheSpec, ModelSpec, StateSpec, TensorSpec
 from ..ops import kernels
 from ..weights import loader
 from ..weights.safetensors_io import CheckpointReader
+from .prompt_layers import PromptLayers
 
 
 class DecoderModel:
@@ -57,6 +58,8 @@ class DecoderModel:
         self.final_norm = build_part("norm", spec.final_norm, rt)
         self.head = build_part("head", spec.head, rt)
         self.nvtx_layers = False           # one NVTX range per layer call (set by the runner from the engine's options)
+        # the plan of prompt steps (None: not this kind of model; False: not looked yet)
+        self._prompt_layers = False
         self._check_order()
 
     # -------------------------------------------------------------- layout
@@ -166,6 +169,11 @@ class DecoderModel:
         residual = ws.get("residual", (rt.max_tokens, self.spec.hidden_size), torch.float32)[:T]
         self.embedding.forward(ctx, residual)
         op_mark(ctx, "embed", nbytes=T * self.spec.hidden_size * (4.0 + (2 if rt.dtype == torch.bfloat16 else 4)))
+        if PromptLayers.takes(ctx) and not self.nvtx_layers:
+            if self._prompt_layers is False:
+                self._prompt_layers = PromptLayers.of(self, caches, ctx)
+            if self._prompt_layers is not None:
+                return residual, self._prompt_layers.run(ctx)
         pending = None
         order = self.spec.order
         embedded = None

@@ -1663,6 +1663,7 @@ def build_all(head_dims=(64, 128), maps_dims=((64, 128, 2), (128, 128, 1)), line
     removes built files of these modules that belong to other versions of the sources."""
     jobs = [(m, f"{m}.cu", None) for m in ("elementwise", "gemm_simt", "gemm_skinny", "gemm_tc", "gemm_mid", "sampling", "rowwise",
                                            "moe", "latent", "stream_ops")]
+    jobs.append(("prompt_layers", "prompt_layers.cpp", None))      # host-only: the launches of a prompt step
     jobs.append(("host_core", "host_core.cpp", None))              # host-only: cache manager, batch filler
     jobs += [(f"attention_d{d}", "attention.cu", {"RL_HEAD_DIM": d}) for d in head_dims]
     for d, v, m, *stride in maps_dims:         # (key size, value size, maps[, length of a value row if longer])
