@@ -85,7 +85,7 @@ static int attend(const RlPromptPlan* p, const RlPromptStep* s, const RlPromptLa
     e = p->attn_decode(kBf16, p->qkv, ld, l.kcache, l.vcache, s->block_table, s->max_blocks, s->decode_info, p->part_o,
                        p->part_ml, s->decode_parts, l.counters, p->attn, out_ld, s->num_decode, p->hq, p->hkv, p->page_size,
                        p->window, p->scale, s->decode_impl, s->stream);
-    ++*launches;
+    *launches += 2;                                     // (the kernel and its merge, as the parts count them)
   }
   if (!e && s->num_tiles > 0) {
     e = p->attn_prefill(kBf16, p->qkv, ld, l.kcache, l.vcache, s->block_table, s->max_blocks, s->tile_seq, s->tile_tok,
