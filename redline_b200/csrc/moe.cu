@@ -634,6 +634,74 @@ moe_gemv_kernel(const T* __restrict__ src, int ld_src, int src_div, const T* __r
   }
 }
 
+// The same where a lane's pieces of a weight row are KI (k = KI x 256 bfloat16 entries or 128 floats): a warp takes NF / (2 if
+// GATED) features and asks for ALL their pieces at once, 16 a lane, 8 KB a warp, together with the tile's rows; the list's
+// entries come in one round trip.  Sums in the order of the kernel above, so the same bits.
+template <typename T, bool GATED, int KI>
+__global__ void __launch_bounds__(128)
+moe_gemv_whole_kernel(const T* __restrict__ src, int ld_src, int src_div, const T* __restrict__ w, int n, int k,
+                      T* __restrict__ dst, int ld_dst, const int32_t* order, const int32_t* tile_expert,
+                      const int32_t* tile_begin, const int32_t* tile_rows, const int32_t* meta, int act, float limit, float slope) {
+  pdl_launch();
+  pdl_wait();
+  constexpr int VEC = Vec16<T>::N, NF = 16 / KI, OF = GATED ? NF / 2 : NF;
+  const int tile = blockIdx.x;
+  const int tiles = meta[0], e = tile_expert[tile], begin = tile_begin[tile], rows = tile_rows[tile];    // (asked for together)
+  if (tile >= tiles) return;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int f0 = (blockIdx.y * 4 + warp) * OF;
+  if (f0 >= n) return;
+  const T* we = w + static_cast<size_t>(e) * (GATED ? 2 * n : n) * k + lane * VEC;
+  uint4 wr[NF][KI];                                // (a feature beyond n: the last one's row, its result is not stored)
+#pragma unroll
+  for (int f = 0; f < NF; ++f) {
+    const T* row = we + (static_cast<size_t>(min(f0 + f % OF, n - 1)) + (f >= OF ? n : 0)) * k;
+#pragma unroll
+    for (int i = 0; i < KI; ++i) wr[f][i] = stream16(row + i * 32 * VEC);
+  }
+  for (int r = 0; r < rows; ++r) {
+    const int pair = order[begin + r];
+    const T* xr = src + static_cast<size_t>(pair / src_div) * ld_src + lane * VEC;
+    uint4 x[KI];
+#pragma unroll
+    for (int i = 0; i < KI; ++i) x[i] = *reinterpret_cast<const uint4*>(xr + i * 32 * VEC);
+    float acc[NF];
+#pragma unroll
+    for (int f = 0; f < NF; ++f) acc[f] = 0.f;
+#pragma unroll
+    for (int i = 0; i < KI; ++i) {
+      float xv[VEC];
+      load16(reinterpret_cast<const T*>(&x[i]), xv);
+#pragma unroll
+      for (int f = 0; f < NF; ++f) {
+        float wv[VEC];
+        load16(reinterpret_cast<const T*>(&wr[f][i]), wv);
+#pragma unroll
+        for (int j = 0; j < VEC; ++j) acc[f] = fmaf(wv[j], xv[j], acc[f]);
+      }
+    }
+#pragma unroll
+    for (int f = 0; f < NF; ++f) acc[f] = warp_sum(acc[f]);
+#pragma unroll
+    for (int f = 0; f < OF; ++f) {
+      float v = acc[f];
+      if (GATED) {
+        const float up = to_float(from_float<T>(acc[f + NF - OF]));
+        v = to_float(from_float<T>(v));
+        if (act == ACT_CLAMPED_SWISH) {
+          const float g = fminf(v, limit);
+          v = g / (1.f + expf(-slope * g)) * (fminf(fmaxf(up, -limit), limit) + 1.f);
+        } else {
+          v = moe_activate(v, act) * up;
+        }
+      } else {
+        v = moe_activate(v, act);
+      }
+      if (lane == 0 && f0 + f < n) dst[static_cast<size_t>(pair) * ld_dst + f0 + f] = from_float<T>(v);
+    }
+  }
+}
+
 // ------------------------------------------------------------------ combine
 // out[t, c] = sum_k weight[t, k] * y[t * top + k, c] (+ shared[t, c])
 template <typename TA>
@@ -727,6 +795,30 @@ int rl_moe_gemm(int act_dtype, const void* src, int ld_src, int src_div, const v
   if (max_tiles <= 0) return 0;
   if (gated && !few_pairs) return static_cast<int>(cudaErrorInvalidValue);
   if (few_pairs) {
+    // (rows of four or eight pieces a lane: 1,024 or 2,048 bfloat16 entries, 512 or 1,024 floats)
+    const int vec = act_dtype == 0 ? 4 : 8;
+    if ((k == 4 * 32 * vec || k == 8 * 32 * vec) && ld_src % vec == 0 && reinterpret_cast<uintptr_t>(src) % 16 == 0 &&
+        reinterpret_cast<uintptr_t>(w) % 16 == 0) {
+      const int ki = k / (32 * vec), of = 4 * (16 / ki) / (gated ? 2 : 1);        // output features of a block
+      const dim3 blocks(max_tiles, (n + of - 1) / of);
+#define RL_CASE(T, G, KI)                                                                                          \
+  launch_kernel(moe_gemv_whole_kernel<T, G, KI>, blocks, dim3(128), 0, stream, static_cast<const T*>(src), ld_src, \
+                src_div, static_cast<const T*>(w), n, k, static_cast<T*>(dst), ld_dst, order, tile_expert,         \
+                tile_begin, tile_rows, meta, act, limit, slope)
+#define RL_SIZES(T, G)                 \
+  do {                                 \
+    if (ki == 4) RL_CASE(T, G, 4);     \
+    else RL_CASE(T, G, 8);             \
+  } while (0)
+      if (act_dtype == 0) {
+        if (gated) RL_SIZES(float, true); else RL_SIZES(float, false);
+      } else {
+        if (gated) RL_SIZES(bf16, true); else RL_SIZES(bf16, false);
+      }
+#undef RL_SIZES
+#undef RL_CASE
+      RL_LAUNCH_END();
+    }
     dim3 g(max_tiles, (n + (gated ? 7 : 15)) / (gated ? 8 : 16));
 #define RL_CASE(T, G)                                                                                              \
   launch_kernel(moe_gemv_kernel<T, G>, g, dim3(128), 0, stream, static_cast<const T*>(src), ld_src, src_div,      \

@@ -1,0 +1,56 @@
+"""Products of a few (token, expert) pairs with a row's weights asked for at once (csrc/moe.cu), and the gated norm
+with the row in registers, against float64.
+
+Tolerances: an output is rounded to bfloat16 once (2^-9 of itself), gate and up once each before the gated form's product;
+float32 sums of up to 4,096 products of order one add 4096^0.5 * 2^-24, nothing beside that: 2^-7 of the largest output."""
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda"
+
+
+@pytest.mark.parametrize("k", [1024, 2048, 2056])
+@pytest.mark.parametrize("gated", [False, True])
+@pytest.mark.parametrize("n,shares", [(16, [1]), (40, [3, 0, 9, 1]), (23, [8, 17, 0, 2, 1])])
+def test_streamed_products(k, gated, n, shares):
+    from redline_b200.ops import kernels
+    E, pairs = len(shares), sum(shares)
+    g = torch.Generator().manual_seed(k + n)
+    x = torch.randn(pairs + 1, k, generator=g).to(torch.bfloat16)
+    w = (torch.randn(E, (2 if gated else 1) * n, k, generator=g) * k ** -0.5).to(torch.bfloat16)
+    expert = torch.tensor([e for e, c in enumerate(shares) for _ in range(c)], dtype=torch.int32)[torch.randperm(pairs, generator=g)]
+    i32 = lambda m: torch.zeros(m, dtype=torch.int32, device=DEV)      # noqa: E731
+    tiles = kernels.moe_max_tiles(pairs, E)
+    order, te, tb, trw, meta = i32(pairs), i32(tiles), i32(tiles), i32(tiles), i32(4)
+    kernels.moe_group(expert.to(DEV), pairs, E, order, te, tb, trw, meta)
+    out = torch.full((pairs, n + 1), float("nan"), dtype=torch.bfloat16, device=DEV)
+    kernels.moe_gemm(x.to(DEV)[:pairs], 1, w.to(DEV).reshape(-1, k), out[:, :n], order, te, tb, trw, meta, tiles,
+                     act=kernels.ACT_SILU, few_pairs=True, gated=gated)
+    y = torch.einsum("pk,pnk->pn", x[:pairs].double(), w[expert.long()].double())
+    if gated:
+        gate, up = (v.to(torch.bfloat16).double() for v in y.split(n, dim=1))
+        want = torch.nn.functional.silu(gate) * up
+    else:
+        want = torch.nn.functional.silu(y)
+    got = out.cpu()
+    assert got[:, n].isnan().all()                       # (nothing beside the columns)
+    assert (got[:, :n].double() - want).abs().max() < 2.0 ** -7 * want.abs().max()
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("rows,n", [(1, 4), (3, 130), (8, 2048), (2, 2049), (5, 4096), (2, 4100)])
+def test_gated_norm(dtype, rows, n):
+    from redline_b200.ops import kernels
+    g = torch.Generator().manual_seed(n)
+    o = torch.randn(rows, n, generator=g)
+    gate = torch.randn(rows, n + 8, generator=g).to(dtype)
+    w = (1.0 + 0.1 * torch.randn(n, generator=g)).to(dtype)
+    out = torch.empty(rows, n, dtype=dtype, device=DEV)
+    kernels.gated_rmsnorm(o.to(DEV), gate.to(DEV)[:, 4:4 + n], w.to(DEV), out, 1e-6)
+    od = o.double()
+    want = od * torch.rsqrt((od * od).mean(-1, keepdim=True) + 1e-6) * w.double() * torch.sigmoid(gate[:, 4:4 + n].double())
+    # (float32: the norm's factor is off by the sum's error, n^0.5 * 2^-24, the rest by a few roundings)
+    tol = (8 + n ** 0.5) * 2.0 ** -24 if dtype == torch.float32 else 2.0 ** -8
+    assert ((out.cpu().double() - want).abs() <= tol * want.abs().max()).all()
