@@ -433,6 +433,43 @@ __global__ void gated_rmsnorm_kernel(const float* __restrict__ o, const TA* __re
   }
 }
 
+// The same with the row in registers, EPT entries per thread (thread t holds t, t + 256, ...), all asked for together and the
+// gate among them: rows are bound by the chain of round trips to memory in steps of few rows, by passes over it in steps of
+// many.  Sums in the order of the kernel above, so the same bits.
+template <typename TA, typename TW, int EPT>
+__global__ void __launch_bounds__(256)
+gated_rmsnorm_reg_kernel(const float* o, const TA* gate, int ld_gate, const TW* __restrict__ w, TA* __restrict__ out, int n,
+                         float eps) {
+  __shared__ float scratch[32];
+  const size_t r = blockIdx.x;
+  const float* orow = o + r * n;
+  const TA* g = gate + r * ld_gate;
+  float wv[EPT], u[EPT], gv[EPT];
+#pragma unroll
+  for (int i = 0; i < EPT; ++i) {          // (the weight comes from no earlier kernel of the step)
+    const int c = threadIdx.x + i * 256;
+    wv[i] = c < n ? to_float(w[c]) : 0.f;
+  }
+  pdl_launch();
+  pdl_wait();
+#pragma unroll
+  for (int i = 0; i < EPT; ++i) {
+    const int c = threadIdx.x + i * 256;
+    u[i] = c < n ? orow[c] : 0.f;
+    gv[i] = c < n ? to_float(g[c]) : 0.f;
+  }
+  float q = 0.f;
+#pragma unroll
+  for (int i = 0; i < EPT; ++i) q += u[i] * u[i];
+  const float rstd = rsqrtf(block_sum(q, scratch) / static_cast<float>(n) + eps);
+#pragma unroll
+  for (int i = 0; i < EPT; ++i) {
+    const int c = threadIdx.x + i * 256;
+    const float s = 1.f / (1.f + expf(-gv[i]));
+    if (c < n) out[r * n + c] = from_float<TA>(u[i] * rstd * wv[i] * s);
+  }
+}
+
 // ------------------------------------------------ u = o * silu(gate);  out = u / rms(u's part) * w
 // The gate first, then the norm of every one of blockIdx.y = 0 .. groups - 1 equal parts of `size` entries by itself.
 // o is the float32 output of a recurrence [T, groups * size].  A part lives in registers, NV pieces of four neighbouring
@@ -846,6 +883,22 @@ int rl_gated_rmsnorm(const float* o, const void* gate, int ld_gate, const void* 
                      int act_dtype, int rows, int n, float eps, cudaStream_t stream) {
   if (rows <= 0) return 0;
   const int th = 256;
+  if (n <= 16 * th) {
+#define RL_CASE(TA, TW)                                                                                               \
+  do {                                                                                                                \
+    if (n <= 8 * th)                                                                                                  \
+      launch_kernel(gated_rmsnorm_reg_kernel<TA, TW, 8>, dim3(rows), dim3(th), 0, stream, o,                          \
+                    static_cast<const TA*>(gate), ld_gate, static_cast<const TW*>(w), static_cast<TA*>(out), n, eps); \
+    else                                                                                                              \
+      launch_kernel(gated_rmsnorm_reg_kernel<TA, TW, 16>, dim3(rows), dim3(th), 0, stream, o,                         \
+                    static_cast<const TA*>(gate), ld_gate, static_cast<const TW*>(w), static_cast<TA*>(out), n, eps); \
+  } while (0)
+    if (act_dtype == RL_F32) RL_CASE(float, float);
+    else if (w_dtype == RL_F32) RL_CASE(bf16, float);
+    else RL_CASE(bf16, bf16);
+#undef RL_CASE
+    RL_LAUNCH_END();
+  }
 #define RL_CASE(TA, TW)                                                                                        \
   launch_kernel(gated_rmsnorm_kernel<TA, TW>, dim3(rows), dim3(th), 0, stream, o, static_cast<const TA*>(gate), \
                 ld_gate, static_cast<const TW*>(w), static_cast<TA*>(out), n, eps)
