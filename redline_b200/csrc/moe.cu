@@ -636,7 +636,9 @@ moe_gemv_kernel(const T* __restrict__ src, int ld_src, int src_div, const T* __r
 
 // The same where a lane's pieces of a weight row are KI (k = KI x 256 bfloat16 entries or 128 floats): a warp takes NF / (2 if
 // GATED) features and asks for ALL their pieces at once, 16 a lane, 8 KB a warp, together with the tile's rows; the list's
-// entries come in one round trip.  Sums in the order of the kernel above, so the same bits.
+// entries come in one round trip.  Sums in the order of the kernel above, so the same bits.  Bound: the weights' way from
+// DRAM.  Eight tokens with four of 32 experts each (about 21 of them, 88 MB): 29.4 us a product with the kernel above,
+// 22.3 (k 2,048, n 1,024) and 23.4 (k 1,024, n 2,048) with this one.
 template <typename T, bool GATED, int KI>
 __global__ void __launch_bounds__(128)
 moe_gemv_whole_kernel(const T* __restrict__ src, int ld_src, int src_div, const T* __restrict__ w, int n, int k,
@@ -795,7 +797,8 @@ int rl_moe_gemm(int act_dtype, const void* src, int ld_src, int src_div, const v
   if (max_tiles <= 0) return 0;
   if (gated && !few_pairs) return static_cast<int>(cudaErrorInvalidValue);
   if (few_pairs) {
-    // (rows of four or eight pieces a lane: 1,024 or 2,048 bfloat16 entries, 512 or 1,024 floats)
+    // rows of four or eight pieces a lane (1,024 or 2,048 bfloat16 entries, 512 or 1,024 floats): with more, 16 pieces a lane
+    // would be one feature a warp, and a gated product needs two
     const int vec = act_dtype == 0 ? 4 : 8;
     if ((k == 4 * 32 * vec || k == 8 * 32 * vec) && ld_src % vec == 0 && reinterpret_cast<uintptr_t>(src) % 16 == 0 &&
         reinterpret_cast<uintptr_t>(w) % 16 == 0) {

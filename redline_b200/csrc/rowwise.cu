@@ -435,7 +435,8 @@ __global__ void gated_rmsnorm_kernel(const float* __restrict__ o, const TA* __re
 
 // The same with the row in registers, EPT entries per thread (thread t holds t, t + 256, ...), all asked for together and the
 // gate among them: rows are bound by the chain of round trips to memory in steps of few rows, by passes over it in steps of
-// many.  Sums in the order of the kernel above, so the same bits.
+// many.  Sums in the order of the kernel above, so the same bits.  Rows of 2,048 in bfloat16: 8 rows 13.0 -> 5.2 us, 1,900 rows
+// 23.8 -> 11.9 (profiled, cold; 31 MB).  Up to 16 entries a thread stay in registers; longer rows take the kernel above.
 template <typename TA, typename TW, int EPT>
 __global__ void __launch_bounds__(256)
 gated_rmsnorm_reg_kernel(const float* o, const TA* gate, int ld_gate, const TW* __restrict__ w, TA* __restrict__ out, int n,
