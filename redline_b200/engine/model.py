@@ -170,10 +170,11 @@ class DecoderModel:
         self.embedding.forward(ctx, residual)
         op_mark(ctx, "embed", nbytes=T * self.spec.hidden_size * (4.0 + (2 if rt.dtype == torch.bfloat16 else 4)))
         if PromptLayers.takes(ctx) and not self.nvtx_layers:
-            if self._prompt_layers is False:
-                self._prompt_layers = PromptLayers.of(self, caches, ctx)
-            if self._prompt_layers is not None:
-                return residual, self._prompt_layers.run(ctx)
+            plan = self._prompt_layers
+            if plan is False or (plan is not None and not plan.fits(self, caches, ctx)):
+                plan = self._prompt_layers = PromptLayers.of(self, caches, ctx)
+            if plan is not None:
+                return residual, plan.run(ctx)
         pending = None
         order = self.spec.order
         embedded = None

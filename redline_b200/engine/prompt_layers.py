@@ -10,11 +10,13 @@ from __future__ import annotations
 import ctypes
 import os
 from ctypes import c_float, c_int, c_int32, c_longlong, c_void_p
+from operator import is_
 from typing import List, Optional
 
 import torch
 
 from ..ops import build, kernels
+from ..parts.base import Watched
 from ..parts.mlp import TC_MIN_ROWS
 from .uniform_layers import uniform_layers
 
@@ -71,8 +73,10 @@ class PromptLayers:
                 (attn, "rl_attn_prefill"), (kernels._lib("gemm_tc", "gemm_tc.cu"), "rl_gemm_tc"),
                 (kernels._lib("gemm_mid", "gemm_mid.cu"), "rl_gemm_mid"), (kernels._ew(), "rl_swiglu")]
         fns = list(library) + [getattr(lib, name) for lib, name in ours]
+        counters = [b.mixer._counters(ctx.max_items) for b in blocks]
+        self.made_at = Watched.last_change                       # (the counters are kept in an attribute)
         rows = [[b.mixer.w_qkv, b.mixer.w_o, b.ffn.w_gate_up, b.ffn.w_down, b.mixer_norm.weight, b.ffn_norm.weight, c.k, c.v,
-                 b.mixer._counters(ctx.max_items)] for b, c in zip(blocks, caches)]
+                 n] for b, c, n in zip(blocks, caches, counters)]
         self.layers = (_Layer * len(rows))(*[_Layer(*[t.data_ptr() for t in row]) for row in rows])
         bf16, f32, mid = torch.bfloat16, torch.float32, kernels.MID_MAX_ROWS
         tiles = kernels.mid_sum_columns(H)
@@ -95,6 +99,26 @@ class PromptLayers:
         self.kept = (rows, buffers, cos, sin, ctx.status)        # what the addresses point at
         self.launch = ctypes.CDLL(build.compile_module("prompt_layers", "prompt_layers.cpp")).rl_prompt_layers
         self.launch.argtypes, self.launch.restype = [c_void_p, c_void_p, c_int, c_void_p], c_int
+        # what ``fits`` compares
+        self.objects = [*blocks, *caches, *(t for c in caches for t in (c.k, c.v))]
+        self.weights = [t for row in rows for t in row[:6]]
+        self.addresses = list(map(torch.Tensor.data_ptr, self.weights))
+        self.sizes = self._sizes(ctx)
+
+    @staticmethod
+    def _sizes(ctx) -> tuple:
+        return ctx.status.data_ptr(), ctx.max_items, ctx.parts_capacity
+
+    def fits(self, model, caches: List[object], ctx) -> bool:
+        """Whether model and step are still what the plan was made for: weights can be loaded again or moved, a part be put
+        in another's place, a method be wrapped, and a step can come with other caches or from another batch builder."""
+        if self.made_at != Watched.last_change or self.sizes != self._sizes(ctx):
+            return False
+        now = [model.blocks[call.layer] for call in model.spec.order]
+        now += caches
+        now += [t for c in caches if c is not None for t in (c.k, c.v)]
+        return (len(now) == len(self.objects) and all(map(is_, self.objects, now))
+                and self.addresses == list(map(torch.Tensor.data_ptr, self.weights)))
 
     @staticmethod
     def takes(ctx) -> bool:

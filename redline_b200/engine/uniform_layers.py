@@ -2,6 +2,7 @@
 
 from __future__ import annotations
 
+from operator import attrgetter
 from typing import List, Optional
 
 import torch
@@ -12,10 +13,17 @@ from ..parts.mlp import SwiGLUMLP
 from ..parts.rmsnorm import RMSNorm
 
 
+# What a step runs of a block and its parts.
+_METHODS = attrgetter("forward", "mixer.forward", "mixer.forward_into", "ffn.forward", "ffn.forward_into", "mixer_norm.add_norm",
+                      "ffn_norm.add_norm")
+_CLASS_METHODS = (PreNormBlock.forward, GQAttention.forward, GQAttention.forward_into, SwiGLUMLP.forward, SwiGLUMLP.forward_into,
+                  RMSNorm.add_norm, RMSNorm.add_norm)
+
+
 def uniform_layers(model, caches: List[object]) -> Optional[list]:
     """The blocks in run order if every one is a pre-norm block of RMSNorm, grouped-query attention with rotary tables
     and a SiLU-gated feed-forward of the same sizes, bfloat16 and without biases, that writes a cache of its own in the
-    same group; None otherwise."""
+    same group; None otherwise, and where one of them has a method of its own (a wrapper around ``forward``, say)."""
     rt, order = model.rt, model.spec.order
     if rt.dtype != torch.bfloat16 or not order:
         return None
@@ -25,6 +33,8 @@ def uniform_layers(model, caches: List[object]) -> Optional[list]:
         if (type(b) is not PreNormBlock or type(b.mixer) is not GQAttention or type(b.ffn) is not SwiGLUMLP
                 or type(b.mixer_norm) is not RMSNorm or type(b.ffn_norm) is not RMSNorm or call.add_embedding
                 or cache is None or not cache.write or cache.group != caches[0].group or not b.ffn.silu):
+            return None
+        if any(getattr(m, "__func__", None) is not of_class for m, of_class in zip(_METHODS(b), _CLASS_METHODS)):
             return None
         att, ffn, a0, f0 = b.mixer, b.ffn, first.mixer, first.ffn
         if any(t is not None for t in (att.b_qkv, att.b_o, ffn.b_gate_up, ffn.b_down)):

@@ -14,6 +14,7 @@ after which a ``PartSpec(kind="my_mixer", ...)`` in a ``ModelSpec`` builds it.
 
 from __future__ import annotations
 
+import itertools
 import os
 from dataclasses import dataclass, field
 from typing import Any, Callable, Dict, List, Optional, Tuple
@@ -125,7 +126,24 @@ class LayerCache:
         return self.tensors["v"]
 
 
-class Part:
+class Watched:
+    """Parts and blocks.  ``Watched.last_change`` is another number after every attribute that is set on any of them (when
+    weights are loaded, a part is put in another's place or a method is wrapped; nothing is set in a step), so that what is
+    made from them knows to be made again."""
+
+    last_change = 0
+    _numbers = itertools.count(1)
+
+    def __setattr__(self, name: str, value: Any) -> None:
+        object.__setattr__(self, name, value)
+        Watched.last_change = next(Watched._numbers)
+
+    def __delattr__(self, name: str) -> None:
+        object.__delattr__(self, name)
+        Watched.last_change = next(Watched._numbers)
+
+
+class Part(Watched):
     def __init__(self, spec: PartSpec, rt: Runtime):
         self.spec = spec
         self.params = spec.params
@@ -325,7 +343,7 @@ class Head(Part):
         return False
 
 
-class Block:
+class Block(Watched):
     """Arrangement of a mixer and a feed-forward around the float32 residual stream.
     ``forward`` gets the stream and a delta that has not been added yet (the previous
     block's last output, so that the add is fused with this block's first norm) and

@@ -39,3 +39,57 @@ def test_the_same_bits_as_part_by_part(name, tmp_path, monkeypatch):
     assert launches["1"] == launches["0"]
     for a, b in zip(outs["1"], outs["0"]):
         assert np.array_equal(a, b)
+
+
+@pytest.mark.parametrize("what", ["weights", "moved", "part", "caches", "builder", "wrapped"])
+def test_a_model_changed_between_steps(what, tmp_path, monkeypatch):
+    """The plan is of the model as it is at the step: after the change, the same bits as part by part."""
+    import torch
+    from redline_b200.cache.storage import CacheStorage
+    from redline_b200.engine.batch import BatchBuilder
+    from redline_b200.weights.safetensors_io import CheckpointReader
+    cfg = C.ALL["tiny_a"]
+    d, _ = make_model(tmp_path / "a", cfg, seed=90)
+    d2, _ = make_model(tmp_path / "b", cfg, seed=91)
+    tokens = [random_tokens(cfg["vocab_size"], 200, 60 + i) for i in range(2)]
+    outs, calls, kept = {}, {"1": 0, "0": 0}, []
+    for mode in ("1", "0"):
+        monkeypatch.setenv("REDLINE_PROMPT_LAYERS", mode)
+        eng = engine_for(d, "bfloat16", kv_cache_tokens=1536)
+        run, model = eng.runner, eng.runner.model
+        eng.step_tokens([("a", tokens[0], [199])])
+        first = model._prompt_layers
+        if what == "weights":
+            model.load_weights(CheckpointReader(d2))
+        elif what == "moved":
+            w = model.blocks[1].ffn.w_down
+            kept.append(w.detach())
+            w.data = -w.data
+        elif what == "part":
+            model.blocks[0], model.blocks[1] = model.blocks[1], model.blocks[0]
+        elif what == "caches":
+            run.storage = CacheStorage(run.groups, [run.storage.of_owner(0, True).k.shape[0]], run.cfg.block_size, run.dtype, run.device)
+            run._caches = [run.storage.of_owner(i, True) for i in range(cfg["num_hidden_layers"])]
+        elif what == "builder":
+            b, c = run.builder, run.cfg
+            run.builder = BatchBuilder(run.cache, c.max_num_batched_tokens, c.max_num_seqs, run.max_rows, c.max_seq_len, run.device,
+                                       b.tile_rows, b.partition)
+            assert run.builder.status.data_ptr() != b.status.data_ptr()
+        else:
+            block, inner = model.blocks[1], model.blocks[1].forward
+
+            def wrapped(*args, mode=mode, inner=inner):
+                calls[mode] += 1
+                return inner(*args)
+            block.forward = wrapped
+        # a prompt in two portions of both kinds, then a token that reads what they left in the cache
+        outs[mode] = [eng.step_tokens([("b", part, [len(part) - 1])]).cpu().numpy()
+                      for part in (tokens[1][:150], tokens[1][150:199], tokens[1][199:])]
+        run.check_status()
+        assert (first is False) == (mode == "0")
+        if what == "builder" and mode == "1":            # (the word in which the step's kernels report belongs to the builder)
+            assert model._prompt_layers is not first
+        torch.cuda.synchronize()
+    for a, b in zip(outs["1"], outs["0"]):
+        assert np.array_equal(a, b)
+    assert calls["1"] == calls["0"]
