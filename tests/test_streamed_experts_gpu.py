@@ -39,14 +39,16 @@ def test_streamed_products(k, gated, n, shares):
     assert (got[:, :n].double() - want).abs().max() < 2.0 ** -7 * want.abs().max()
 
 
-@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
-@pytest.mark.parametrize("rows,n", [(1, 4), (3, 130), (8, 2048), (2, 2049), (5, 4096), (2, 4100)])
-def test_gated_norm(dtype, rows, n):
+@pytest.mark.parametrize("dtype,w_dtype", [(torch.float32, torch.float32), (torch.bfloat16, torch.bfloat16),
+                                           (torch.bfloat16, torch.float32)])
+@pytest.mark.parametrize("rows,n", [(1, 4), (3, 130), (2, 256), (2, 257), (3, 512), (2, 513), (2, 1024), (2, 1025), (8, 2048),
+                                    (2, 2049), (5, 4096), (2, 4100)])
+def test_gated_norm(dtype, w_dtype, rows, n):
     from redline_b200.ops import kernels
     g = torch.Generator().manual_seed(n)
     o = torch.randn(rows, n, generator=g)
     gate = torch.randn(rows, n + 8, generator=g).to(dtype)
-    w = (1.0 + 0.1 * torch.randn(n, generator=g)).to(dtype)
+    w = (1.0 + 0.1 * torch.randn(n, generator=g)).to(w_dtype)
     out = torch.empty(rows, n, dtype=dtype, device=DEV)
     kernels.gated_rmsnorm(o.to(DEV), gate.to(DEV)[:, 4:4 + n], w.to(DEV), out, 1e-6)
     od = o.double()
