@@ -798,12 +798,13 @@ int rl_moe_gemm(int act_dtype, const void* src, int ld_src, int src_div, const v
   if (gated && !few_pairs) return static_cast<int>(cudaErrorInvalidValue);
   if (few_pairs) {
     // rows of four or eight pieces a lane (1,024 or 2,048 bfloat16 entries, 512 or 1,024 floats): with more, 16 pieces a lane
-    // would be one feature a warp, and a gated product needs two
-    const int vec = act_dtype == 0 ? 4 : 8;
-    if ((k == 4 * 32 * vec || k == 8 * 32 * vec) && ld_src % vec == 0 && reinterpret_cast<uintptr_t>(src) % 16 == 0 &&
-        reinterpret_cast<uintptr_t>(w) % 16 == 0) {
-      const int ki = k / (32 * vec), of = 4 * (16 / ki) / (gated ? 2 : 1);        // output features of a block
-      const dim3 blocks(max_tiles, (n + of - 1) / of);
+    // would be one feature a warp, and a gated product needs two; other lengths have not been tried.  (A grid has no more
+    // than 65,535 blocks in y.)
+    const int vec = act_dtype == 0 ? 4 : 8, per_block = k == 8 * 32 * vec ? (gated ? 4 : 8) : (gated ? 8 : 16);
+    if ((k == 4 * 32 * vec || k == 8 * 32 * vec) && (n + per_block - 1) / per_block <= 65535 && ld_src % vec == 0 &&
+        reinterpret_cast<uintptr_t>(src) % 16 == 0 && reinterpret_cast<uintptr_t>(w) % 16 == 0) {
+      const int ki = k / (32 * vec);
+      const dim3 blocks(max_tiles, (n + per_block - 1) / per_block);        // (per_block: output features of a block)
 #define RL_CASE(T, G, KI)                                                                                          \
   launch_kernel(moe_gemv_whole_kernel<T, G, KI>, blocks, dim3(128), 0, stream, static_cast<const T*>(src), ld_src, \
                 src_div, static_cast<const T*>(w), n, k, static_cast<T*>(dst), ld_dst, order, tile_expert,         \

@@ -39,6 +39,22 @@ def test_streamed_products(k, gated, n, shares):
     assert (got[:, :n].double() - want).abs().max() < 2.0 ** -7 * want.abs().max()
 
 
+def test_streamed_products_of_many_features():
+    """An expert whose features are more than the grid has blocks for with four of them each."""
+    from redline_b200.ops import kernels
+    n, k, rows = 4 * 65535 + 8, 2048, 3
+    g = torch.Generator(device=DEV).manual_seed(5)
+    x = torch.randn(rows, k, generator=g, device=DEV).to(torch.bfloat16)
+    w = torch.empty(2 * n, k, dtype=torch.bfloat16, device=DEV).normal_(0.0, k ** -0.5, generator=g)
+    out = torch.empty(rows, n, dtype=torch.bfloat16, device=DEV)
+    i32 = lambda *v: torch.tensor(v, dtype=torch.int32, device=DEV)    # noqa: E731
+    kernels.moe_gemm(x, 1, w, out, i32(0, 1, 2), i32(0), i32(0), i32(rows), i32(1, 0, 0, 0), 1, act=kernels.ACT_SILU,
+                     few_pairs=True, gated=True)
+    gate, up = x.float() @ w[n - 32:n].float().t(), x.float() @ w[2 * n - 32:].float().t()
+    want = torch.nn.functional.silu(gate.to(torch.bfloat16).float()) * up.to(torch.bfloat16).float()
+    assert (out[:, n - 32:].float() - want).abs().max() < 2.0 ** -7 * want.abs().max()
+
+
 @pytest.mark.parametrize("dtype,w_dtype", [(torch.float32, torch.float32), (torch.bfloat16, torch.bfloat16),
                                            (torch.bfloat16, torch.float32)])
 @pytest.mark.parametrize("rows,n", [(1, 4), (3, 130), (2, 256), (2, 257), (3, 512), (2, 513), (2, 1024), (2, 1025), (8, 2048),
