@@ -635,12 +635,22 @@ moe_gemv_kernel(const T* __restrict__ src, int ld_src, int src_div, const T* __r
 }
 
 // The same where a lane's pieces of a weight row are KI (k = KI x 256 bfloat16 entries or 128 floats): a warp takes NF / (2 if
-// GATED) features and asks for ALL their pieces at once, 16 a lane, 8 KB a warp, together with the tile's rows; the list's
-// entries come in one round trip.  Sums in the order of the kernel above, so the same bits.  Bound: the weights' way from
-// DRAM.  Eight tokens with four of 32 experts each (about 21 of them, 88 MB): 29.4 us a product with the kernel above,
-// 22.3 (k 2,048, n 1,024) and 23.4 (k 1,024, n 2,048) with this one.
-template <typename T, bool GATED, int KI>
-__global__ void __launch_bounds__(128)
+// GATED) features and asks for ALL their pieces at once, 16 a lane, 8 KB a warp.  Sums in the order of the kernel above, so the
+// same bits.  Bound: the weights' way from DRAM where experts have a few rows, a row's chain (list, entries, sums, the warp's
+// sum) where they have many.  AHEAD: 32 entries of the list at once and the next row's entries before the present one's sums.
+// That is for bfloat16 at KI 4 and floats at KI 8; the others have no registers for it: three CTAs an SM are worth more at
+// KI 8 in bfloat16 (with two, 64 experts of a row 60 us instead of 47), five at KI 4 in float32 (with four, 32 of two rows 29
+// instead of 24).  us a product with the kernel above / with this one, by experts x rows of each (k, output features):
+//                            64 x 1      21 x 2      16 x 4      8 x 8       4 x 16      1 x 64
+//   bfloat16 2,048, 1,024   83.8/47.2   37.2/22.9   31.9/27.3   30.9/26.9   54.2/32.2    185/59
+//     gated                  142/85.4   52.9/37.8   49.7/43.0   54.1/39.0   50.4/42.5    185/56
+//   bfloat16 1,024, 2,048    118/46.8   42.8/23.7   36.5/28.9   35.9/28.8   35.4/34.0    123/65
+//     gated, 512            50.6/24.4   22.2/12.7   18.7/15.4   17.5/16.1   30.6/16.0    105/48
+//   float32 1,024, gated     120/75.0   44.0/27.6   40.2/29.2   49.0/26.1   46.5/25.3    163/44
+//   float32 512, 2,048       113/39.3   41.1/17.2   34.2/20.8   32.5/22.2   30.8/21.2    109/63
+// (Without AHEAD the third row's 4 x 16 took 39.1 and the fourth one's 8 x 8 19.6.)
+template <typename T, bool GATED, int KI, bool AHEAD = (KI == 8) == (sizeof(T) == 4)>
+__global__ void __launch_bounds__(128, KI == 4 && sizeof(T) == 4 ? 0 : 3)
 moe_gemv_whole_kernel(const T* __restrict__ src, int ld_src, int src_div, const T* __restrict__ w, int n, int k,
                       T* __restrict__ dst, int ld_dst, const int32_t* order, const int32_t* tile_expert,
                       const int32_t* tile_begin, const int32_t* tile_rows, const int32_t* meta, int act, float limit, float slope) {
@@ -661,12 +671,32 @@ moe_gemv_whole_kernel(const T* __restrict__ src, int ld_src, int src_div, const 
 #pragma unroll
     for (int i = 0; i < KI; ++i) wr[f][i] = stream16(row + i * 32 * VEC);
   }
-  for (int r = 0; r < rows; ++r) {
-    const int pair = order[begin + r];
+  auto ask = [&](int pair, uint4 (&to)[KI]) {
     const T* xr = src + static_cast<size_t>(pair / src_div) * ld_src + lane * VEC;
-    uint4 x[KI];
 #pragma unroll
-    for (int i = 0; i < KI; ++i) x[i] = *reinterpret_cast<const uint4*>(xr + i * 32 * VEC);
+    for (int i = 0; i < KI; ++i) to[i] = *reinterpret_cast<const uint4*>(xr + i * 32 * VEC);
+  };
+  int listed = 0, next = 0;                        // (AHEAD) 32 entries of the tile's list, the one of the next row
+  uint4 ahead[KI];
+  if (AHEAD) {
+    listed = lane < rows ? order[begin + lane] : 0;
+    next = __shfl_sync(0xffffffffu, listed, 0);
+    ask(next, ahead);
+  }
+  for (int r = 0; r < rows; ++r) {
+    const int pair = AHEAD ? next : order[begin + r];
+    uint4 x[KI];
+    if (AHEAD) {
+#pragma unroll
+      for (int i = 0; i < KI; ++i) x[i] = ahead[i];
+      if (r + 1 < rows) {
+        if ((r + 1) % 32 == 0 && r + 1 + lane < rows) listed = order[begin + r + 1 + lane];
+        next = __shfl_sync(0xffffffffu, listed, (r + 1) % 32);
+        ask(next, ahead);
+      }
+    } else {
+      ask(pair, x);
+    }
     float acc[NF];
 #pragma unroll
     for (int f = 0; f < NF; ++f) acc[f] = 0.f;

@@ -11,32 +11,52 @@ pytestmark = pytest.mark.gpu
 DEV = "cuda"
 
 
-@pytest.mark.parametrize("k", [1024, 2048, 2056])
-@pytest.mark.parametrize("gated", [False, True])
-@pytest.mark.parametrize("n,shares", [(16, [1]), (40, [3, 0, 9, 1]), (23, [8, 17, 0, 2, 1])])
-def test_streamed_products(k, gated, n, shares):
+def product(x, src_div, w, expert, n, act, gated, limit=0.0, slope=1.0):
+    """The experts' product of pairs listed in ``expert`` (x, w on the CPU); one column more than asked for, of NaN."""
     from redline_b200.ops import kernels
-    E, pairs = len(shares), sum(shares)
-    g = torch.Generator().manual_seed(k + n)
-    x = torch.randn(pairs + 1, k, generator=g).to(torch.bfloat16)
-    w = (torch.randn(E, (2 if gated else 1) * n, k, generator=g) * k ** -0.5).to(torch.bfloat16)
-    expert = torch.tensor([e for e, c in enumerate(shares) for _ in range(c)], dtype=torch.int32)[torch.randperm(pairs, generator=g)]
+    E, pairs = w.shape[0], expert.numel()
     i32 = lambda m: torch.zeros(m, dtype=torch.int32, device=DEV)      # noqa: E731
     tiles = kernels.moe_max_tiles(pairs, E)
     order, te, tb, trw, meta = i32(pairs), i32(tiles), i32(tiles), i32(tiles), i32(4)
     kernels.moe_group(expert.to(DEV), pairs, E, order, te, tb, trw, meta)
-    out = torch.full((pairs, n + 1), float("nan"), dtype=torch.bfloat16, device=DEV)
-    kernels.moe_gemm(x.to(DEV)[:pairs], 1, w.to(DEV).reshape(-1, k), out[:, :n], order, te, tb, trw, meta, tiles,
-                     act=kernels.ACT_SILU, few_pairs=True, gated=gated)
-    y = torch.einsum("pk,pnk->pn", x[:pairs].double(), w[expert.long()].double())
+    out = torch.full((pairs, n + 1), float("nan"), dtype=x.dtype, device=DEV)
+    kernels.moe_gemm(x.to(DEV), src_div, w.to(DEV).reshape(-1, x.shape[1]), out[:, :n], order, te, tb, trw, meta, tiles,
+                     act=act, few_pairs=True, gated=gated, limit=limit, slope=slope)
+    return out.cpu()
+
+
+@pytest.mark.parametrize("dtype,k", [(torch.bfloat16, 1024), (torch.bfloat16, 2048), (torch.bfloat16, 2056),
+                                     (torch.float32, 512), (torch.float32, 1024), (torch.float32, 516)])
+@pytest.mark.parametrize("gated,act", [(False, "silu"), (True, "silu"), (True, "clamped_swish")])
+@pytest.mark.parametrize("n,shares,top", [(16, [1], 1), (40, [3, 0, 9, 1], 1), (23, [8, 17, 0, 2, 1], 4), (9, [1, 33, 0, 130], 2)])
+def test_streamed_products(dtype, k, gated, act, n, shares, top):
+    """Against float64, and bit for bit against the kernel for any length: rows and weights with zeros behind them go there,
+    and its sums are these in the same order."""
+    from redline_b200.ops import kernels
+    E, pairs, limit, slope = len(shares), sum(shares), 1.5, 1.25
+    g = torch.Generator().manual_seed(k + n)
+    x = torch.randn((pairs + top - 1) // top, k, generator=g).to(dtype)
+    w = (torch.randn(E, (2 if gated else 1) * n, k, generator=g) * k ** -0.5).to(dtype)
+    expert = torch.tensor([e for e, c in enumerate(shares) for _ in range(c)], dtype=torch.int32)[torch.randperm(pairs, generator=g)]
+    code = kernels.ACT_CLAMPED_SWISH if act == "clamped_swish" else kernels.ACT_SILU
+    got = product(x, top, w, expert, n, code, gated, limit, slope)
+    y = torch.einsum("pk,pnk->pn", x[torch.arange(pairs) // top].double(), w[expert.long()].double())
     if gated:
-        gate, up = (v.to(torch.bfloat16).double() for v in y.split(n, dim=1))
-        want = torch.nn.functional.silu(gate) * up
+        gate, up = (v.to(dtype).double() for v in y.split(n, dim=1))
+        if act == "clamped_swish":
+            gate = gate.clamp(max=limit)
+            want = gate * torch.sigmoid(slope * gate) * (up.clamp(-limit, limit) + 1.0)
+        else:
+            want = torch.nn.functional.silu(gate) * up
     else:
         want = torch.nn.functional.silu(y)
-    got = out.cpu()
     assert got[:, n].isnan().all()                       # (nothing beside the columns)
-    assert (got[:, :n].double() - want).abs().max() < 2.0 ** -7 * want.abs().max()
+    # (float32: sums of k products of order k^-0.5, each rounded, and a few roundings more)
+    tol = 2.0 ** -7 if dtype == torch.bfloat16 else (8 + k ** 0.5) * 2.0 ** -24
+    assert (got[:, :n].double() - want).abs().max() < tol * want.abs().max()
+    more = 256 if dtype == torch.bfloat16 else 128
+    pad = lambda t: torch.nn.functional.pad(t, (0, 5 * more))          # noqa: E731
+    assert torch.equal(product(pad(x), top, pad(w), expert, n, code, gated, limit, slope)[:, :n], got[:, :n])
 
 
 def test_streamed_products_of_many_features():
