@@ -42,6 +42,15 @@ class _Step(ctypes.Structure):
     _fields_ += [(n, c_int32) for n in ("T", "max_blocks", "num_decode", "decode_parts", "num_tiles", "decode_impl")]
 
 
+class _Counts(ctypes.Structure):
+    _fields_ = [("launches", c_int32), ("failed", c_int32)]
+
+
+# The plan's launchers by the names that their errors have elsewhere.
+_LAUNCHERS = ("cublasGemmEx", "cublasSetMathMode", "add_rmsnorm", "rope_kv_write", "attn_decode", "attn_prefill", "gemm_tc",
+              "gemm_mid", "swiglu")
+
+
 def _library(name: str):
     """A function of the cuBLAS that torch has loaded, or None."""
     try:
@@ -136,9 +145,9 @@ class PromptLayers:
                      g.slots.data_ptr(), g.block_table.data_ptr(), ctx.decode_info.data_ptr(), ctx.tile_seq.data_ptr(),
                      ctx.tile_tok.data_ptr(), ctx.tile_rows.data_ptr(), ctx.T, g.block_table.shape[1], ctx.num_decode,
                      ctx.decode_parts, ctx.num_tiles, self.mixer.decode_variant(ctx) if ctx.num_decode > 0 else 0)
-        n = c_int(0)
+        n = _Counts()
         code = self.launch(ctypes.addressof(self.plan), ctypes.addressof(step), 1 if few else 0, ctypes.addressof(n))
-        if code >= 100000:
-            raise kernels.KernelError(f"prompt_layers: cuBLAS status {code - 100000}")
-        kernels._check(code, "prompt_layers", n.value)
+        if code != 0 and n.failed < 2:
+            raise kernels.KernelError(f"{_LAUNCHERS[n.failed]}: cuBLAS status {code}")
+        kernels._check(code, _LAUNCHERS[n.failed], n.launches)
         return None if few else self.ffn_out[:ctx.T]
