@@ -9,6 +9,7 @@ from __future__ import annotations
 
 import ctypes
 import os
+import warnings
 from ctypes import c_float, c_int, c_int32, c_longlong, c_void_p
 from operator import is_
 from typing import List, Optional
@@ -52,10 +53,12 @@ _LAUNCHERS = ("cublasGemmEx", "cublasSetMathMode", "add_rmsnorm", "rope_kv_write
 
 
 def _library(name: str):
-    """A function of the cuBLAS that torch has loaded, or None."""
+    """A function of the cuBLAS that torch has loaded, or None, with a warning (torch without it)."""
+    soname = f"libcublas.so.{(torch.version.cuda or '').split('.')[0]}"
     try:
-        return getattr(ctypes.CDLL("libcublas.so.12", mode=os.RTLD_NOLOAD | os.RTLD_NOW), name)
+        return getattr(ctypes.CDLL(soname, mode=os.RTLD_NOLOAD | os.RTLD_NOW), name)
     except (OSError, AttributeError):
+        warnings.warn(f"{soname} is not loaded or has no {name}: the layers of prompt steps are launched from Python")
         return None
 
 
@@ -64,11 +67,13 @@ class PromptLayers:
     def of(model, caches: List[object], ctx) -> Optional["PromptLayers"]:
         """The plan for this model with these caches, or None if its layers are not alike."""
         blocks = uniform_layers(model, caches)
-        fns = [_library("cublasGemmEx"), _library("cublasSetMathMode")]
-        if blocks is None or None in fns:
+        if blocks is None:
             return None
         p = blocks[0].mixer.params
         if p.hidden_size % 8 or blocks[0].ffn.params.intermediate_size % 8:
+            return None
+        fns = [_library("cublasGemmEx"), _library("cublasSetMathMode")]
+        if None in fns:
             return None
         return PromptLayers(model, blocks, caches, ctx, fns)
 

@@ -53,3 +53,17 @@ def test_a_failed_launch_is_the_one_named(T, num_decode):
         assert got == 700 + i and PL._LAUNCHERS[n.failed] == name
         back = ["cublasSetMathMode"] if many and 0 < i < len(called) - 1 else []
         assert some == called[:i + 1] + back
+
+
+def test_the_library_of_another_torch(monkeypatch):
+    """The library is looked for by the CUDA version that torch was built for; one that is not there is told of."""
+    asked = []
+
+    def nothing(name, mode):
+        asked.append(name)
+        raise OSError(name)
+    monkeypatch.setattr(PL.ctypes, "CDLL", nothing)
+    monkeypatch.setattr(PL.torch.version, "cuda", "13.1")
+    with pytest.warns(UserWarning, match="libcublas.so.13"):
+        assert PL._library("cublasGemmEx") is None
+    assert asked == ["libcublas.so.13"]
