@@ -6,12 +6,20 @@ import pytest
 
 import tiny_configs as C
 from gpu_utils import engine_for, make_model, random_tokens
+from test_parts_gpu import engine_from_spec, spec_with
 
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("name", ["tiny_a", "tiny_b"])
-def test_the_same_bits_as_part_by_part(name, tmp_path, monkeypatch):
+def engine(d, cfg, window, **kw):
+    if not window:
+        return engine_for(d, "bfloat16", kv_cache_tokens=1536, **kw)
+    return engine_from_spec(d, cfg, spec_with(cfg, window=window), "bfloat16", kv_cache_tokens=1536, **kw)
+
+
+@pytest.mark.parametrize("name,window", [("tiny_a", 0), ("tiny_b", 0), ("tiny_c", 0), ("tiny_a", 40)])
+def test_the_same_bits_as_part_by_part(name, window, tmp_path, monkeypatch):
+    from redline_b200.engine.prompt_layers import PromptLayers
     from redline_b200.ops import kernels
     cfg = C.ALL[name]
     d, _ = make_model(tmp_path, cfg, seed=90)
@@ -24,7 +32,7 @@ def test_the_same_bits_as_part_by_part(name, tmp_path, monkeypatch):
     outs, launches = {}, {}
     for mode in ("1", "0"):
         monkeypatch.setenv("REDLINE_PROMPT_LAYERS", mode)
-        eng = engine_for(d, "bfloat16", kv_cache_tokens=1536)
+        eng = engine(d, cfg, window)
         at, outs[mode], launches[mode] = {0: 0, 1: 0, 2: 0}, [], []
         for step in steps:
             entries = []
@@ -34,9 +42,31 @@ def test_the_same_bits_as_part_by_part(name, tmp_path, monkeypatch):
             before = kernels.LAUNCHES
             outs[mode].append(eng.step_tokens(entries).cpu().numpy())
             launches[mode].append(kernels.LAUNCHES - before)
-        assert (eng.runner.model._prompt_layers is False) == (mode == "0")
+        plan = eng.runner.model._prompt_layers
+        assert isinstance(plan, PromptLayers) if mode == "1" else plan is False
         eng.runner.check_status()
     assert launches["1"] == launches["0"]
+    for a, b in zip(outs["1"], outs["0"]):
+        assert np.array_equal(a, b)
+
+
+@pytest.mark.parametrize("window", [0, 40])
+def test_full_portions_as_a_graph(window, tmp_path, monkeypatch):
+    """Full portions of a prompt are captured once and replayed for the next ones; the rest of the prompt runs eagerly."""
+    from redline_b200.engine.prompt_layers import PromptLayers
+    cfg = C.ALL["tiny_a"]
+    d, _ = make_model(tmp_path, cfg, seed=92)
+    tokens = random_tokens(cfg["vocab_size"], 128 * 3 + 70, 33)
+    outs = {}
+    for mode in ("1", "0"):
+        monkeypatch.setenv("REDLINE_PROMPT_LAYERS", mode)
+        eng = engine(d, cfg, window, cuda_graphs=True, max_num_batched_tokens=128)
+        outs[mode] = [eng.step_tokens([("a", tokens[i:i + 128], [min(128, len(tokens) - i) - 1])], graphs=True).cpu().numpy()
+                      for i in range(0, len(tokens), 128)]
+        assert eng.runner.num_graph_steps == 3 and eng.runner.num_eager_steps == 1 and len(eng.runner._graphs) == 1
+        plan = eng.runner.model._prompt_layers
+        assert isinstance(plan, PromptLayers) if mode == "1" else plan is False
+        eng.runner.check_status()
     for a, b in zip(outs["1"], outs["0"]):
         assert np.array_equal(a, b)
 
@@ -47,6 +77,7 @@ def test_a_model_changed_between_steps(what, tmp_path, monkeypatch):
     import torch
     from redline_b200.cache.storage import CacheStorage
     from redline_b200.engine.batch import BatchBuilder
+    from redline_b200.engine.prompt_layers import PromptLayers
     from redline_b200.weights.safetensors_io import CheckpointReader
     cfg = C.ALL["tiny_a"]
     d, _ = make_model(tmp_path / "a", cfg, seed=90)
@@ -86,7 +117,7 @@ def test_a_model_changed_between_steps(what, tmp_path, monkeypatch):
         outs[mode] = [eng.step_tokens([("b", part, [len(part) - 1])]).cpu().numpy()
                       for part in (tokens[1][:150], tokens[1][150:199], tokens[1][199:])]
         run.check_status()
-        assert (first is False) == (mode == "0")
+        assert isinstance(first, PromptLayers) if mode == "1" else first is False
         if what == "builder" and mode == "1":            # (the word in which the step's kernels report belongs to the builder)
             assert model._prompt_layers is not first
         torch.cuda.synchronize()
