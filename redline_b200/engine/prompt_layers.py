@@ -16,7 +16,7 @@ from typing import List, Optional
 
 import torch
 
-from ..ops import build, kernels
+from ..ops import kernels
 from ..parts.base import Watched
 from ..parts.mlp import TC_MIN_ROWS
 from .uniform_layers import uniform_layers
@@ -111,10 +111,10 @@ class PromptLayers:
                           len(rows), H, I, p.num_heads, p.num_kv_heads, p.head_dim, rt.page_size, p.window, cos.shape[0],
                           kernels.sm_count(rt.device), TC_MIN_ROWS, tiles)
         self.kept = (rows, buffers, cos, sin, ctx.status)        # what the addresses point at
-        self.launch = ctypes.CDLL(build.compile_module("prompt_layers", "prompt_layers.cpp")).rl_prompt_layers
-        self.launch.argtypes, self.launch.restype = [c_void_p, c_void_p, c_int, c_void_p], c_int
+        self.launch = kernels._fn(kernels._lib("prompt_layers", "prompt_layers.cpp"), "rl_prompt_layers",
+                                  [c_void_p, c_void_p, c_int, c_void_p])
         # what ``fits`` compares
-        self.objects = [*blocks, *caches, *(t for c in caches for t in (c.k, c.v))]
+        self.spec, self.blocks, self.caches = model.spec, list(model.blocks), list(caches)
         self.weights = [t for row in rows for t in row[:6]]
         self.addresses = list(map(torch.Tensor.data_ptr, self.weights))
         self.sizes = self._sizes(ctx)
@@ -126,12 +126,9 @@ class PromptLayers:
     def fits(self, model, caches: List[object], ctx) -> bool:
         """Whether model and step are still what the plan was made for: weights can be loaded again or moved, a part be put
         in another's place, a method be wrapped, and a step can come with other caches or from another batch builder."""
-        if self.made_at != Watched.last_change or self.sizes != self._sizes(ctx):
-            return False
-        now = [model.blocks[call.layer] for call in model.spec.order]
-        now += caches
-        now += [t for c in caches if c is not None for t in (c.k, c.v)]
-        return (len(now) == len(self.objects) and all(map(is_, self.objects, now))
+        return (self.made_at == Watched.last_change and self.sizes == self._sizes(ctx) and self.spec is model.spec
+                and len(self.blocks) == len(model.blocks) and all(map(is_, self.blocks, model.blocks))
+                and len(self.caches) == len(caches) and all(map(is_, self.caches, caches))
                 and self.addresses == list(map(torch.Tensor.data_ptr, self.weights)))
 
     @staticmethod

@@ -46,10 +46,11 @@ def _fn(lib: ctypes.CDLL, name: str, argtypes):
     return f
 
 
-# A prompt step launches 140 kernels from Python and is as long as that takes unless it is large, so these helpers
-# stay out of torch's Python layers: a stream handle by ``torch.cuda.current_stream()`` alone was 7 us of the 20 us
-# that a launch took, pointers wrapped in c_void_p another 2 (plain integers do as well).  A prompt of 333 tokens
-# went from 3.06 to 1.98 ms with them and the workspace's kept views.
+# A step whose layers are launched part by part (prompts of most designs, steps of single tokens without graphs) is as
+# long as its launches from Python take unless it is large, so these helpers stay out of torch's Python layers: a stream
+# handle by ``torch.cuda.current_stream()`` alone was 7 us of the 20 us that a launch took, pointers wrapped in c_void_p
+# another 2 (plain integers do as well).  A prompt of 333 tokens in a 1B model, 140 launches then, went from 3.06 to
+# 1.98 ms with them and the workspace's kept views.
 # (A torch without CUDA has neither function: the module still imports there, and a launch says why it cannot be.)
 def _no_cuda(*_):
     raise KernelError("redline_b200 kernels need a torch that was built with CUDA")
