@@ -94,7 +94,6 @@ class PromptLayers:
         self.layers = (_Layer * len(rows))(*[_Layer(*[t.data_ptr() for t in row]) for row in rows])
         bf16, f32, mid = torch.bfloat16, torch.float32, kernels.MID_MAX_ROWS
         tiles = kernels.mid_sum_columns(H)
-        parts = ctx.max_items * p.num_heads * ctx.parts_capacity
         # (the buffers that the parts use, by the same names)
         self.residual = ws.get("residual", (T, H), f32)
         self.ffn_out = ws.get("ffn.out", (T, H), bf16)
@@ -102,11 +101,10 @@ class PromptLayers:
                    ws.get("attn.out", (T, att.q_size), bf16), ws.get("mixer.out", (T, H), bf16), ws.get("ffn.act", (T, I), bf16),
                    ws.get("ffn.gate_up", (min(T, TC_MIN_ROWS), 2 * I), bf16), self.ffn_out,
                    ws.get("attn.mid.hand_xw", (mid, H), bf16), ws.get("ffn.mid.hand_xw", (mid, H), bf16),
-                   ws.get("attn.mid.hand_sums", (mid, tiles), f32), ws.get("ffn.mid.hand_sums", (mid, tiles), f32),
-                   ws.get("attn.part_o", (parts * p.head_dim,), f32), ws.get("attn.part_ml", (parts * 2,), f32)]
+                   ws.get("attn.mid.hand_sums", (mid, tiles), f32), ws.get("ffn.mid.hand_sums", (mid, tiles), f32)]
         cos, sin = att.position.rotary_tables()
         self.plan = _Plan(*[ctypes.cast(f, c_void_p).value for f in fns], ctypes.addressof(self.layers),
-                          *[t.data_ptr() for t in buffers], cos.data_ptr(), sin.data_ptr(), ctx.status.data_ptr(),
+                          *[t.data_ptr() for t in buffers], None, None, cos.data_ptr(), sin.data_ptr(), ctx.status.data_ptr(),
                           kernels.tc_status(rt.device).data_ptr(), caches[0].k.shape[0] * rt.page_size, norm.params.eps, att.scale,
                           len(rows), H, I, p.num_heads, p.num_kv_heads, p.head_dim, rt.page_size, p.window, cos.shape[0],
                           kernels.sm_count(rt.device), TC_MIN_ROWS, tiles)
@@ -143,6 +141,12 @@ class PromptLayers:
         """Takes the step's embeddings in the stream's buffer through all layers; returns what is still to be added to the
         stream (None: nothing)."""
         g, few = ctx.groups[self.group], ctx.T <= kernels.MID_ROUTED_ROWS
+        if ctx.num_decode > 0 and not self.plan.part_o:
+            # (asked for by the first step with single tokens: 2 GB for 256 sequences of up to 131,072 tokens with 32 heads)
+            ws, p = self.rt.workspace, self.mixer.params
+            n = ctx.max_items * p.num_heads * ctx.parts_capacity
+            self.parts = ws.get("attn.part_o", (n * p.head_dim,), torch.float32), ws.get("attn.part_ml", (n * 2,), torch.float32)
+            self.plan.part_o, self.plan.part_ml = (t.data_ptr() for t in self.parts)
         step = _Step(0 if few else torch.cuda.current_blas_handle(), kernels._stream(), ctx.positions.data_ptr(),
                      g.slots.data_ptr(), g.block_table.data_ptr(), ctx.decode_info.data_ptr(), ctx.tile_seq.data_ptr(),
                      ctx.tile_tok.data_ptr(), ctx.tile_rows.data_ptr(), ctx.T, g.block_table.shape[1], ctx.num_decode,

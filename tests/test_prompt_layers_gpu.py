@@ -124,3 +124,18 @@ def test_a_model_changed_between_steps(what, tmp_path, monkeypatch):
     for a, b in zip(outs["1"], outs["0"]):
         assert np.array_equal(a, b)
     assert calls["1"] == calls["0"]
+
+
+def test_no_workspace_for_single_tokens_before_there_are_some(tmp_path):
+    """The partial results of decode attention, which grow with sequences and their length, are not asked for by prompts."""
+    import torch
+    cfg = C.ALL["tiny_a"]
+    d, _ = make_model(tmp_path, cfg, seed=93)
+    eng = engine(d, cfg, 0)
+    held = eng.runner.rt.workspace._bufs
+    for steps in ([("a", [5] * 150, [149])], [("a", [6] * 40, [39]), ("b", [7] * 20, [19])]):
+        eng.step_tokens(steps)
+        assert ("attn.part_o", torch.float32) not in held and ("attn.part_ml", torch.float32) not in held
+    eng.step_tokens([("a", [8], [0]), ("b", [9] * 30, [29])])
+    assert ("attn.part_o", torch.float32) in held and ("attn.part_ml", torch.float32) in held
+    eng.runner.check_status()
