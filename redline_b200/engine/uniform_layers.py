@@ -2,7 +2,8 @@
 
 from __future__ import annotations
 
-from operator import attrgetter
+from functools import lru_cache
+from inspect import isfunction
 from typing import List, Optional
 
 import torch
@@ -13,17 +14,24 @@ from ..parts.mlp import SwiGLUMLP
 from ..parts.rmsnorm import RMSNorm
 
 
-# What a step runs of a block and its parts.
-_METHODS = attrgetter("forward", "mixer.forward", "mixer.forward_into", "ffn.forward", "ffn.forward_into", "mixer_norm.add_norm",
-                      "ffn_norm.add_norm")
-_CLASS_METHODS = (PreNormBlock.forward, GQAttention.forward, GQAttention.forward_into, SwiGLUMLP.forward, SwiGLUMLP.forward_into,
-                  RMSNorm.add_norm, RMSNorm.add_norm)
+@lru_cache(maxsize=None)
+def _methods(kind: type) -> tuple:
+    found = {}
+    for k in reversed(kind.__mro__):
+        found.update((name, f) for name, f in vars(k).items() if isfunction(f))
+    return tuple(found.items())
+
+
+def _own_method(part) -> bool:
+    """Whether the object has a method of its own in place of its class's (a wrapper around ``forward``, say).  (Asked by
+    attribute: a look into an object's ``__dict__`` would make its attributes slower for good.)"""
+    return any(getattr(getattr(part, name), "__func__", None) is not f for name, f in _methods(type(part)))
 
 
 def uniform_layers(model, caches: List[object]) -> Optional[list]:
     """The blocks in run order if every one is a pre-norm block of RMSNorm, grouped-query attention with rotary tables
     and a SiLU-gated feed-forward of the same sizes, bfloat16 and without biases, that writes a cache of its own in the
-    same group; None otherwise, and where one of them has a method of its own (a wrapper around ``forward``, say)."""
+    same group; None otherwise, and where one of them has a method of its own."""
     rt, order = model.rt, model.spec.order
     if rt.dtype != torch.bfloat16 or not order:
         return None
@@ -34,7 +42,7 @@ def uniform_layers(model, caches: List[object]) -> Optional[list]:
                 or type(b.mixer_norm) is not RMSNorm or type(b.ffn_norm) is not RMSNorm or call.add_embedding
                 or cache is None or not cache.write or cache.group != caches[0].group or not b.ffn.silu):
             return None
-        if any(getattr(m, "__func__", None) is not of_class for m, of_class in zip(_METHODS(b), _CLASS_METHODS)):
+        if any(map(_own_method, (b, b.mixer, b.mixer.position, b.ffn, b.mixer_norm, b.ffn_norm))):
             return None
         att, ffn, a0, f0 = b.mixer, b.ffn, first.mixer, first.ffn
         if any(t is not None for t in (att.b_qkv, att.b_o, ffn.b_gate_up, ffn.b_down)):

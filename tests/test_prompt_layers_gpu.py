@@ -71,7 +71,7 @@ def test_full_portions_as_a_graph(window, tmp_path, monkeypatch):
         assert np.array_equal(a, b)
 
 
-@pytest.mark.parametrize("what", ["weights", "moved", "part", "caches", "builder", "wrapped"])
+@pytest.mark.parametrize("what", ["weights", "moved", "part", "caches", "builder", "forward", "_attend"])
 def test_a_model_changed_between_steps(what, tmp_path, monkeypatch):
     """The plan is of the model as it is at the step: after the change, the same bits as part by part."""
     import torch
@@ -107,12 +107,13 @@ def test_a_model_changed_between_steps(what, tmp_path, monkeypatch):
                                        b.tile_rows, b.partition)
             assert run.builder.status.data_ptr() != b.status.data_ptr()
         else:
-            block, inner = model.blocks[1], model.blocks[1].forward
+            part = model.blocks[1] if what == "forward" else model.blocks[1].mixer
+            inner = getattr(part, what)
 
             def wrapped(*args, mode=mode, inner=inner):
                 calls[mode] += 1
                 return inner(*args)
-            block.forward = wrapped
+            setattr(part, what, wrapped)
         # a prompt in two portions of both kinds, then a token that reads what they left in the cache
         outs[mode] = [eng.step_tokens([("b", part, [len(part) - 1])]).cpu().numpy()
                       for part in (tokens[1][:150], tokens[1][150:199], tokens[1][199:])]
@@ -123,7 +124,7 @@ def test_a_model_changed_between_steps(what, tmp_path, monkeypatch):
         torch.cuda.synchronize()
     for a, b in zip(outs["1"], outs["0"]):
         assert np.array_equal(a, b)
-    assert calls["1"] == calls["0"]
+    assert calls["1"] == calls["0"] == (3 if what in ("forward", "_attend") else 0)
 
 
 def test_no_workspace_for_single_tokens_before_there_are_some(tmp_path):
